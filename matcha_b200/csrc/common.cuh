@@ -36,6 +36,32 @@ __host__ __device__ inline int mtb_dsize(int L) {
   return L < 0 ? 0 : (L + 1) * (2 * L + 1) * (2 * L + 3) / 3;
 }
 
+// Launch with clusters of `cluster` CTAs along x (grid.x a multiple of it).
+template <typename... Args>
+inline cudaError_t launch_clusters(void (*kernel)(Args...), dim3 grid, int block, size_t smem, int cluster,
+                                   cudaStream_t st, Args... args) {
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = (unsigned)cluster;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3((unsigned)block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
+// CTAs that share one subtomogram of a batch of B: the smallest power of two up to 8 that gives
+// an SM about `per_sm` CTAs.  More would only repeat each CTA's prologue.
+inline int cluster_size(int B, int per_sm) {
+  int s = 1;
+  while (s < 8 && (int64_t)B * s < (int64_t)per_sm * 148) s *= 2;
+  return s;
+}
+
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

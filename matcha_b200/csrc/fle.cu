@@ -300,6 +300,7 @@ struct mtb_fle {
   int* koff;
   int* kidx;
   int kmax;      // max over degrees of kpad
+  int* kpad_host;  // kpad on the host
   FleTc tc;
   bool use_tc;
 };
@@ -368,7 +369,11 @@ extern "C" int mtb_fle_create(const mtb_fle_config* cfg, mtb_fle** out) {
   std::vector<int> koff(L + 1);
   int kt = 0;
   for (int l = 0; l <= L; ++l) { koff[l] = kt; kt += (2 * l + 1) * cfg->kpad[l]; }
-  for (int l = 0; l <= L; ++l) h->kmax = cfg->kpad[l] > h->kmax ? cfg->kpad[l] : h->kmax;
+  h->kpad_host = new int[L + 1];
+  for (int l = 0; l <= L; ++l) {
+    h->kmax = cfg->kpad[l] > h->kmax ? cfg->kpad[l] : h->kmax;
+    h->kpad_host[l] = cfg->kpad[l];
+  }
   for (int i = 0; i < kt; ++i)
     if (cfg->kidx[i] >= cfg->ne) return fail(MTB_ERR_ARG);
 
@@ -452,6 +457,7 @@ extern "C" void mtb_fle_destroy(mtb_fle* h) {
   void* ptrs[] = {h->d_basis, h->d_class_cols, h->d_class_off, h->rep_img, h->col_re, h->col_im, h->s_re, h->s_im,
                   h->A, h->C, h->kpad, h->koff, h->kidx};
   for (void* p : ptrs) if (p) cudaFree(p);
+  delete[] h->kpad_host;
   delete h;
 }
 
@@ -521,13 +527,14 @@ extern "C" int mtb_sigma(mtb_fle* h, const float* coeffs, int64_t coeff_stride, 
 
 // The sigma gather tables of a handle, for the template backward (backward.cu).
 int fle_sigma_tables(const mtb_fle* h, const int** kpad, const int** koff, const int** kidx, int* lmax, int* kmax,
-                     int* ne) {
+                     int* ne, const int** kpad_host) {
   *kpad = h->kpad;
   *koff = h->koff;
   *kidx = h->kidx;
   *lmax = h->cfg.lmax;
   *kmax = h->kmax;
   *ne = h->cfg.ne;
+  *kpad_host = h->kpad_host;
   return MTB_OK;
 }
 
