@@ -24,6 +24,7 @@
 #include <stdio.h>
 #include <string.h>
 #include <vector>
+#include <cooperative_groups.h>
 #include <cuda_bf16.h>
 #include "common.cuh"
 #include "shift_tc.cuh"
@@ -1650,50 +1651,88 @@ __global__ void finalize_kernel(ShiftGeom g, int B, int ngrp, const float* __res
 //   fftfreq(N)[m1], fftfreq(N/2+1)[m2]),
 // the function whose values on the grid s = (u - dftshift) / uf the upsampled DFT evaluates
 // (ShiftMatcher.py:46-91, with the half axis taken as a full period as there), and
-// dc/ds_d = -2 pi sum_m f_d(m) Im(P[m] exp(2 pi i s . f(m))) / (|T| |S|).  One CTA per
-// subtomogram; s and the gradient in (x, y, z) order like the shifts the search returns.
-__device__ __forceinline__ float fftfreq_of(int m, int n) { return (float)(m <= (n - 1) / 2 ? m : m - n) / (float)n; }
+// dc/ds_d = -2 pi sum_m f_d(m) Im(P[m] exp(2 pi i s . f(m))) / (|T| |S|); s and the gradient in
+// (x, y, z) order like the shifts the search returns.
+//
+// Bound by reading P once.  The phase is a product of one factor per axis, tabulated in FP64, so
+// an element costs one complex multiply-add per sum instead of a sincos: a thread owns columns
+// (m1, m2) and adds P e0[m0] and P f0 e0[m0] along m0 in FP64 (eight independent loads in flight),
+// and the factors e1 e2 and the frequencies of the other axes meet the two sums once per column.
+// The planes m0 of a subtomogram are split over the CTAs of a cluster, whose four sums meet
+// through distributed shared memory in rank order (deterministic).  256 subtomograms of 64^3
+// (277 MB): 109 us, against 578 us with one CTA per subtomogram and a sincos per element.
+__device__ __forceinline__ double fftfreq_of(int m, int n) { return (double)(m <= (n - 1) / 2 ? m : m - n) / (double)n; }
 
 __global__ void __launch_bounds__(256)
 shift_score_grad_kernel(ShiftGeom g, const float2* __restrict__ P, const float* __restrict__ nrm,
                         const float* __restrict__ s_xyz, float* __restrict__ score, float* __restrict__ grad_xyz) {
-  const int b = blockIdx.x;
-  const int N = g.N, H = g.H;
-  const int64_t per = (int64_t)N * N * H;
-  const float2* p = P + (int64_t)b * per;
-  const float sx = s_xyz[3 * b + 0], sy = s_xyz[3 * b + 1], sz = s_xyz[3 * b + 2];
-  double v = 0.0, gx = 0.0, gy = 0.0, gz = 0.0;
-  for (int64_t e = threadIdx.x; e < per; e += blockDim.x) {
-    const int m0 = (int)(e / ((int64_t)N * H)), m1 = (int)((e / H) % N), m2 = (int)(e % H);
-    const float fz = fftfreq_of(m0, N), fy = fftfreq_of(m1, N), fx = fftfreq_of(m2, H);
-    float sn, cs;
-    sincospif(2.f * (sz * fz + sy * fy + sx * fx), &sn, &cs);
-    const float2 q = p[e];
-    const float re = q.x * cs - q.y * sn, im = q.x * sn + q.y * cs;
-    v += re;
-    gx += (double)(fx * im);
-    gy += (double)(fy * im);
-    gz += (double)(fz * im);
+  namespace cg = cooperative_groups;
+  cg::cluster_group cluster = cg::this_cluster();
+  const int rank = (int)cluster.block_rank(), parts = (int)cluster.num_blocks(), b = blockIdx.y;
+  const int N = g.N, H = g.H, NC = N * H;
+  __shared__ double2 e0[128], e1[128], e2[65];  // e^{2 pi i s f(m)} per axis (z, y, x), N <= 128
+  __shared__ double f0[128];
+  __shared__ double red[4][8], sum[4];
+  for (int t = threadIdx.x; t < 2 * N + H; t += blockDim.x) {
+    const int ax = t < N ? 0 : (t < 2 * N ? 1 : 2), m = t - ax * N;
+    const double f = fftfreq_of(m, ax == 2 ? H : N);
+    double sn, cs;
+    sincospi(2.0 * (double)s_xyz[3 * b + 2 - ax] * f, &sn, &cs);
+    (ax == 0 ? e0 : (ax == 1 ? e1 : e2))[m] = make_double2(cs, sn);
+    if (ax == 0) f0[m] = f;
   }
-  __shared__ double red[4][256];
-  red[0][threadIdx.x] = v;
-  red[1][threadIdx.x] = gx;
-  red[2][threadIdx.x] = gy;
-  red[3][threadIdx.x] = gz;
   __syncthreads();
-  for (int s = 128; s > 0; s >>= 1) {
-    if ((int)threadIdx.x < s)
-      for (int k = 0; k < 4; ++k) red[k][threadIdx.x] += red[k][threadIdx.x + s];
-    __syncthreads();
+  const int per = (N + parts - 1) / parts, lo = rank * per, hi = min(N, lo + per);
+  const float2* p = P + (int64_t)b * N * NC;
+  double v = 0.0, gx = 0.0, gy = 0.0, gz = 0.0;
+  for (int c = threadIdx.x; c < NC; c += blockDim.x) {
+    double rr = 0.0, ri = 0.0, zr = 0.0, zi = 0.0;  // sums of P e0 and of P f0 e0
+#pragma unroll 8
+    for (int m0 = lo; m0 < hi; ++m0) {
+      const float2 q = __ldg(p + (int64_t)m0 * NC + c);
+      const double2 e = e0[m0];
+      const double f = f0[m0];
+      const double tr = (double)q.x * e.x - (double)q.y * e.y, ti = (double)q.x * e.y + (double)q.y * e.x;
+      rr += tr;
+      ri += ti;
+      zr = fma(f, tr, zr);
+      zi = fma(f, ti, zi);
+    }
+    const int m1 = c / H, m2 = c - (c / H) * H;
+    const double2 a = e1[m1], d = e2[m2];
+    const double wr = a.x * d.x - a.y * d.y, wi = a.x * d.y + a.y * d.x;
+    const double im = rr * wi + ri * wr;
+    v += rr * wr - ri * wi;
+    gx += fftfreq_of(m2, H) * im;
+    gy += fftfreq_of(m1, N) * im;
+    gz += zr * wi + zi * wr;
   }
-  if (threadIdx.x == 0) {
+  double x[4] = {v, gx, gy, gz};
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) x[k] += __shfl_xor_sync(0xffffffffu, x[k], o);
+    if (lane == 0) red[k][warp] = x[k];
+  }
+  __syncthreads();
+  if (threadIdx.x < 4) {
+    double s = 0.0;
+    for (int q = 0; q < 8; ++q) s += red[threadIdx.x][q];
+    sum[threadIdx.x] = s;
+  }
+  cluster.sync();
+  if (rank == 0 && threadIdx.x < 4) {
+    const int k = threadIdx.x;
+    double s = 0.0;
+    for (int q = 0; q < parts; ++q) s += cluster.map_shared_rank(&sum[k], q)[0];
     const double den = sqrt((double)nrm[2 * b]) * sqrt((double)nrm[2 * b + 1]);
-    const double tp = -2.0 * 3.14159265358979323846 / den;
-    score[b] = (float)(red[0][0] / den);
-    grad_xyz[3 * b + 0] = (float)(tp * red[1][0]);
-    grad_xyz[3 * b + 1] = (float)(tp * red[2][0]);
-    grad_xyz[3 * b + 2] = (float)(tp * red[3][0]);
+    if (k == 0)
+      score[b] = (float)(s / den);
+    else
+      grad_xyz[3 * b + k - 1] = (float)(-2.0 * 3.14159265358979323846 / den * s);
   }
+  cluster.sync();  // no CTA leaves while its sums are read
 }
 
 // Tensor-core path: decode the per-subtomogram argmax key of the third pass.
@@ -2164,8 +2203,9 @@ extern "C" int mtb_shift_score_grad(mtb_shift* h, const float* subtomos, const f
   // the FP32 product in T, whatever the handle's precision
   if (int rc = shift_front(h, subtomos, shift_zyx, rot, ctf, B, st, false)) return rc;
   mtb_prof_begin(st);
-  shift_score_grad_kernel<<<B, 256, 0, st>>>(h->g, reinterpret_cast<const float2*>(h->T), h->nrm, query_xyz, score,
-                                             grad_xyz);
+  const int parts = cluster_size(B, 4);
+  MTB_CUDA_TRY(launch_clusters(shift_score_grad_kernel, dim3(parts, B), 256, 0, parts, st, h->g,
+                               (const float2*)h->T, (const float*)h->nrm, query_xyz, score, grad_xyz));
   mtb_prof_end(st, "shift_score_grad_kernel");
   MTB_LAUNCH_CHECK();
   return MTB_OK;
