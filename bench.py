@@ -297,7 +297,7 @@ def kernel_work(B):
         "gemm_tc_kernel": ("tensor", 2.0 * n_rep * n_cols),
         "expand_kernel": ("hbm", 4 * n_cols + 8 * ne),
         "sigma_kernel": ("hbm", 8 * ne + 8 * dsize(L_MAX)),
-        "so3_grid_topk_kernel": ("hbm", 8 * dsize(8)),
+        "so3_grid_columns_kernel": ("hbm", 8 * dsize(8)),
         "fold_sigma_kernel": ("hbm", 8 * dsize(L_MAX) + 16 * sum((l + 1) ** 2 for l in range(L_MAX + 1))),
         "tracker_update_kernel": ("hbm", 3 * 4 + 2 * 32 + 36),
         "patch_fft_xy64_kernel": ("hbm", vol + spec),

@@ -7,7 +7,8 @@
 //   D, d      src/matcha/core/WignerDMatrices.py:281-306, 673-801, 1291-1375
 //   g, H      src/matcha/core/WignerDGradients.py:155-302
 //
-// Design (B200): one CTA per (subtomogram, candidate) runs every march stage for
+// Design (B200): the grid runs in grid.cu (oversampling 2) or the general kernel here;
+// one CTA per (subtomogram, candidate) runs every march stage for
 // its candidate.  The small-d matrix of each degree l is produced by the three-term
 // recurrence in l for fixed (m', m) (state in registers, one fundamental wedge
 // m' >= |m| per thread, symmetric copies written to shared memory), and contracted
@@ -20,6 +21,7 @@
 #include <string.h>
 #include <vector>
 #include "common.cuh"
+#include "grid.cuh"
 #include "newton.cuh"
 
 namespace {
@@ -98,18 +100,14 @@ size_t grid_smem_bytes(int L0, int K) {
 //   G_j[m'][g] = sum_m F_j[m'][m] e^{2 pi i g m / n}
 //   f_j[a][g]  = Re sum_{m'} G_j[m'][g] e^{2 pi i a m' / n} / n^2
 // with the running top-C of every thread merged at the end.
-// L0T, NT > 0 fix L0 and n at compile time (the index arithmetic then folds to constants);
-// 0 takes them from the arguments.  KC >= C is the capacity of each thread's kept set, held
-// in registers (statically indexed).
-template <int L0T, int NT, int KC, bool STAGED>
+// KC >= C is the capacity of each thread's kept set, held in registers (statically indexed).
+template <int KC, bool STAGED>
 __global__ void __launch_bounds__(kGridThreads)
 so3_grid_topk_kernel(const float2* __restrict__ sigma, int64_t stride, int B,
-                     const float* __restrict__ dtab, int L0_arg, int n_arg, int C, int JB,
+                     const float* __restrict__ dtab, int L0, int n, int C, int JB,
                      float* __restrict__ alpha, float* __restrict__ beta, float* __restrict__ gamma,
                      float* __restrict__ grid_out) {
   extern __shared__ __align__(16) float gsm[];
-  const int L0 = L0T > 0 ? L0T : L0_arg;
-  const int n = NT > 0 ? NT : n_arg;
   const int P = 2 * L0 - 1;
   const int nk = mtb_dsize(L0 - 1);
   float2* sg = reinterpret_cast<float2*>(gsm);  // nk
@@ -169,61 +167,27 @@ so3_grid_topk_kernel(const float2* __restrict__ sigma, int64_t stride, int B,
       const int l0 = max(abs(mp), abs(m));
       const float* dj = STAGED ? sD + jb * nk : dtab + (int64_t)(j0 + jb) * nk;
       float re = 0.f, im = 0.f;
-      if (L0T > 0) {
-#pragma unroll
-        for (int l = 0; l < L0T; ++l) {
-          if (l >= l0) {
-            const int idx = mtb_dsize(l - 1) + (mp + l) * (2 * l + 1) + (m + l);
-            const float d = STAGED ? dj[idx] : __ldg(dj + idx);
-            re += d * sg[idx].x;
-            im += d * sg[idx].y;
-          }
-        }
-      } else {
-        for (int l = l0; l < L0; ++l) {
-          const int idx = mtb_dsize(l - 1) + (mp + l) * (2 * l + 1) + (m + l);
-          const float d = STAGED ? dj[idx] : __ldg(dj + idx);
-          re += d * sg[idx].x;
-          im += d * sg[idx].y;
-        }
+      for (int l = l0; l < L0; ++l) {
+        const int idx = mtb_dsize(l - 1) + (mp + l) * (2 * l + 1) + (m + l);
+        const float d = STAGED ? dj[idx] : __ldg(dj + idx);
+        re += d * sg[idx].x;
+        im += d * sg[idx].y;
       }
       F[q] = make_float2(re, im);
     }
     __syncthreads();
-    if constexpr (NT > 0) {
-      // four outputs gg = g4 + (n/4) i per thread: one F read serves four independent chains
-      constexpr int n4 = NT / 4;
-      for (int q = tid; q < jn * P * n4; q += blockDim.x) {
-        const int jb = q / (P * n4), qq = q - jb * (P * n4);
-        const int r = qq / n4, g4 = qq - (qq / n4) * n4;
-        const float2* fr = F + jb * P * P + r * P;
-        float re[4] = {0.f, 0.f, 0.f, 0.f}, im[4] = {0.f, 0.f, 0.f, 0.f};
-        for (int c = 0; c < P; ++c) {
-          const float2 f = fr[c];
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const float2 t = TW[(g4 + n4 * i) * P + c];
-            re[i] += f.x * t.x - f.y * t.y;
-            im[i] += f.x * t.y + f.y * t.x;
-          }
-        }
-#pragma unroll
-        for (int i = 0; i < 4; ++i) G[jb * P * n + r * n + g4 + n4 * i] = make_float2(re[i], im[i]);
+    for (int q = tid; q < jn * P * n; q += blockDim.x) {
+      const int jb = q / (P * n), qq = q - jb * (P * n);
+      const int r = qq / n, gg = qq - (qq / n) * n;
+      const float2* fr = F + jb * P * P + r * P;
+      const float2* tr = TW + gg * P;
+      float re = 0.f, im = 0.f;
+      for (int c = 0; c < P; ++c) {
+        const float2 f = fr[c], t = tr[c];
+        re += f.x * t.x - f.y * t.y;
+        im += f.x * t.y + f.y * t.x;
       }
-    } else {
-      for (int q = tid; q < jn * P * n; q += blockDim.x) {
-        const int jb = q / (P * n), qq = q - jb * (P * n);
-        const int r = qq / n, gg = qq - (qq / n) * n;
-        const float2* fr = F + jb * P * P + r * P;
-        const float2* tr = TW + gg * P;
-        float re = 0.f, im = 0.f;
-        for (int c = 0; c < P; ++c) {
-          const float2 f = fr[c], t = tr[c];
-          re += f.x * t.x - f.y * t.y;
-          im += f.x * t.y + f.y * t.x;
-        }
-        G[q] = make_float2(re, im);
-      }
+      G[q] = make_float2(re, im);
     }
     __syncthreads();
     // offer one grid value to this thread's kept set
@@ -242,40 +206,17 @@ so3_grid_topk_kernel(const float2* __restrict__ sigma, int64_t stride, int B,
         if (cnt == C) find_min();
       }
     };
-    if constexpr (NT > 0) {
-      // four outputs gg = g4 + (n/4) i per thread: one twiddle read serves four chains (the
-      // kept set is a total order on (value, index), so the visiting order does not matter)
-      constexpr int n4 = NT / 4;
-      for (int q = tid; q < jn * n * n4; q += blockDim.x) {
-        const int jb = q / (n * n4), qq = q - jb * (n * n4);
-        const int aa = qq / n4, g4 = qq - (qq / n4) * n4;
-        const float2* gc = G + jb * P * n + g4;
-        const float2* ta = TW + aa * P;
-        float re[4] = {0.f, 0.f, 0.f, 0.f};
-        for (int r = 0; r < P; ++r) {
-          const float2 t = ta[r];
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const float2 gv = gc[r * n + n4 * i];
-            re[i] += gv.x * t.x - gv.y * t.y;
-          }
-        }
-#pragma unroll
-        for (int i = 0; i < 4; ++i) offer(re[i] * inv_n2, (j0 + jb) * n * n + aa * n + g4 + n4 * i);
+    for (int q = tid; q < jn * n * n; q += blockDim.x) {
+      const int jb = q / (n * n), qq = q - jb * (n * n);
+      const int aa = qq / n, gg = qq - (qq / n) * n;
+      const float2* gc = G + jb * P * n + gg;
+      const float2* ta = TW + aa * P;
+      float re = 0.f;
+      for (int r = 0; r < P; ++r) {
+        const float2 gv = gc[r * n], t = ta[r];
+        re += gv.x * t.x - gv.y * t.y;
       }
-    } else {
-      for (int q = tid; q < jn * n * n; q += blockDim.x) {
-        const int jb = q / (n * n), qq = q - jb * (n * n);
-        const int aa = qq / n, gg = qq - (qq / n) * n;
-        const float2* gc = G + jb * P * n + gg;
-        const float2* ta = TW + aa * P;
-        float re = 0.f;
-        for (int r = 0; r < P; ++r) {
-          const float2 gv = gc[r * n], t = ta[r];
-          re += gv.x * t.x - gv.y * t.y;
-        }
-        offer(re * inv_n2, (j0 + jb) * n * n + qq);
-      }
+      offer(re * inv_n2, (j0 + jb) * n * n + qq);
     }
     __syncthreads();
   }
@@ -324,21 +265,21 @@ so3_grid_topk_kernel(const float2* __restrict__ sigma, int64_t stride, int B,
   }
 }
 
-template <int L0T, int NT, int KC>
+template <int KC>
 int grid_launch_t(const float2* sigma, int64_t stride, int B, const float* dtab, int L0, int K, int C, float* a,
                   float* b, float* g, float* grid, cudaStream_t st) {
   const size_t smem = grid_smem_bytes(L0, K);
   const int jb = grid_jb(L0, K);
   mtb_prof_begin(st);
   if (grid_staged(L0, K)) {
-    MTB_CUDA_TRY(cudaFuncSetAttribute(so3_grid_topk_kernel<L0T, NT, KC, true>,
+    MTB_CUDA_TRY(cudaFuncSetAttribute(so3_grid_topk_kernel<KC, true>,
                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    so3_grid_topk_kernel<L0T, NT, KC, true><<<B, kGridThreads, smem, st>>>(sigma, stride, B, dtab, L0, 2 * L0 * K,
+    so3_grid_topk_kernel<KC, true><<<B, kGridThreads, smem, st>>>(sigma, stride, B, dtab, L0, 2 * L0 * K,
                                                                        C, jb, a, b, g, grid);
   } else {
-    MTB_CUDA_TRY(cudaFuncSetAttribute(so3_grid_topk_kernel<L0T, NT, KC, false>,
+    MTB_CUDA_TRY(cudaFuncSetAttribute(so3_grid_topk_kernel<KC, false>,
                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    so3_grid_topk_kernel<L0T, NT, KC, false><<<B, kGridThreads, smem, st>>>(sigma, stride, B, dtab, L0, 2 * L0 * K,
+    so3_grid_topk_kernel<KC, false><<<B, kGridThreads, smem, st>>>(sigma, stride, B, dtab, L0, 2 * L0 * K,
                                                                         C, jb, a, b, g, grid);
   }
   mtb_prof_end(st, "so3_grid_topk_kernel");
@@ -346,18 +287,16 @@ int grid_launch_t(const float2* sigma, int64_t stride, int B, const float* dtab,
   return MTB_OK;
 }
 
-// The grid search for L0 = 8, 12, 16 with K = 2 (the marches of boxes 64, 96 and 128 at
-// bandlimit N/2) with its index arithmetic fixed at compile time; other grids take the general
-// instantiation.
+// The grid search.  The column kernel takes oversampling 2 from L0 = 3 to 16 (every march the
+// configurations use; larger L0 would not keep a column in registers); other grids take the
+// general kernel.  Both give the same grid bit by bit.  An instantiation of the general kernel with its indexes fixed
+// at compile time took 421 us for 1000 subtomograms at L0 = 8 and 1207 us for 64 at L0 = 16, the
+// column kernel takes 193 and 239 us.
 int grid_launch(const float2* sigma, int64_t stride, int B, const float* dtab, int L0, int K, int C, float* a,
                 float* b, float* g, float* grid, cudaStream_t st) {
-  if (L0 == 8 && K == 2 && C <= 16) return grid_launch_t<8, 32, 16>(sigma, stride, B, dtab, L0, K, C, a, b, g, grid, st);
-  if (L0 == 12 && K == 2 && C <= 16)
-    return grid_launch_t<12, 48, 16>(sigma, stride, B, dtab, L0, K, C, a, b, g, grid, st);
-  if (L0 == 16 && K == 2 && C <= 16)
-    return grid_launch_t<16, 64, 16>(sigma, stride, B, dtab, L0, K, C, a, b, g, grid, st);
-  if (C <= 16) return grid_launch_t<0, 0, 16>(sigma, stride, B, dtab, L0, K, C, a, b, g, grid, st);
-  return grid_launch_t<0, 0, kMaxCand>(sigma, stride, B, dtab, L0, K, C, a, b, g, grid, st);
+  if (grid_columns_cover(L0, K)) return grid_columns_launch(sigma, stride, B, dtab, L0, C, a, b, g, grid, st);
+  if (C <= 16) return grid_launch_t<16>(sigma, stride, B, dtab, L0, K, C, a, b, g, grid, st);
+  return grid_launch_t<kMaxCand>(sigma, stride, B, dtab, L0, K, C, a, b, g, grid, st);
 }
 
 __global__ void reduce_candidates_kernel(const float* __restrict__ ca, const float* __restrict__ cb,
