@@ -3,11 +3,19 @@
 // The 8 octant-parity GEMMs of fle.cu, C_p = A_p * B_p (A: folded volumes, B: basis
 // columns), run here as BF16 x BF16 -> FP32 products with a split correction:
 //     A B ~= A_hi B_hi + A_lo B_hi + A_hi B_lo,   A_hi = bf16(A), A_lo = bf16(A - A_hi)
-// (the dropped A_lo B_lo term is ~2^-16 relative).  The three products are one GEMM over
-// a K axis three times as long: k-block j of [0, 3 KB) selects (A_hi, B_hi), (A_lo, B_hi)
-// or (A_hi, B_lo), so every pipeline stage moves one A tile and one B tile.  (Staging the
-// hi and lo tiles of both operands per K block, 96 KB, leaves room for two stages only,
-// which measured 2.2x slower: the loads are no longer hidden.)
+// (the dropped A_lo B_lo term is ~2^-16 relative).  Two orders of the products, by the basis:
+//   segmented    one GEMM over a K axis three times as long: step j of [0, 3 KB) selects (A_hi,
+//                B_hi), (A_lo, B_hi) or (A_hi, B_lo), so a pipeline stage moves one tile of each,
+//                64 along K.
+//   interleaved  a stage holds the hi and lo tiles of both operands, 32 along K, for all three
+//                products: the same bytes per stage, two thirds of the bytes per product, and B_hi
+//                read once instead of twice.  (With stages of 64 along K only two fit, which was
+//                1242 against 1187 us on the second line below and 2.2x slower on the first.)
+// The second is for a basis that does not stay in L2 (64^3 up: 500 MB), where the loads, into
+// shared memory and from DRAM, set the pace; below, where the whole GEMM takes tens of us, the
+// first.  Times of the GEMM, before (segmented, one CTA per tile) and now: 1000 subtomograms of
+// 64^3 679 -> 545 us (1.47 PFLOP/s issued), 100 of 96^3 1397 -> 1187 us (5.1 TB/s of basis), 256 of
+// 64^3 324 -> 223 us, one of 48^3 85 -> 37 us.
 //
 // Accumulation: the tensor core adds each K=16 product into the FP32 accumulator with a
 // truncating alignment, an error of about one unit in the last place of the accumulator per
@@ -20,13 +28,20 @@
 // the other buffer; C is written once at the end.  (Adding each chunk into C in global memory
 // instead measured 2.4x slower: one row per lane makes every access a 32-way scatter.)
 //
-// Layout: both operands K-major bf16, 128-byte swizzled tiles staged by TMA
-// (cp.async.bulk.tensor.2d), tile M = 128 (a batch block), N = 256 (basis columns),
-// K = 64 per stage, 4 stages of 48 KB.  One thread issues tcgen05.mma (kind::f16, M128 N256
-// K16); eight warps read the accumulators back with tcgen05.ld, two per 32-lane quarter of
-// tensor memory, each keeping 128 columns of its row.  A and B of all classes and
-// both parts share two tensor maps: rows (class * 2 + part) * Mpad + m of A,
-// (class * 2 + part) * Npad + n of B.
+// Layout: both operands K-major bf16, tiles with 128-byte (interleaved: 64-byte) swizzle staged by
+// TMA (cp.async.bulk.tensor.2d), tile M = 128 (a batch block), N = 256 or less (the basis columns of
+// a class cut evenly, to 16).  One thread issues tcgen05.mma (kind::f16, M128 K16);
+// eight warps read the accumulators back with tcgen05.ld, two per 32-lane quarter of tensor
+// memory, each keeping 128 columns of its row.  A has rows (class * 2 + part) * Mpad + m; B is
+// stored tile by tile, [class][part][N tile][K block][column][64], so that a stage's tile is one
+// contiguous run of DRAM (with a K row per column instead, 1266 against 1242 us for 100
+// subtomograms of 96^3).
+//
+// Work units: the tiles that fill whole rounds of the 148 SMs are one CTA each; the rest are cut
+// along K into parts of q chunks (gemm_plan).  The first part of a tile leaves its sums in C, the
+// others leave theirs in slabs (one per chunk, or one per part in the interleaved order), and the
+// part that arrives last adds the slabs to C in order.  With a slab per chunk the additions are
+// those of a whole tile, so a coefficient does not depend on the split, nor on the batch it is in.
 //
 // Every mbarrier wait is bounded; on expiry the kernel records an error code, stops
 // issuing, waits (bounded) for the MMAs it issued, and frees its tensor memory before
@@ -44,73 +59,88 @@ namespace {
 using namespace tc;
 
 constexpr int TM = 128, TN = 256, TK = 64;
-constexpr int STAGES = 4;
+constexpr int kMaxStages = 8;
 constexpr int A_TILE = TM * TK * 2;  // 16 KB
-constexpr int B_TILE = TN * TK * 2;  // 32 KB
-constexpr int STAGE_BYTES = A_TILE + B_TILE;
+constexpr int TKI = 32;              // K of a stage in the interleaved order
+constexpr int AI_TILE = TM * TKI * 2;
+constexpr size_t kSmemCap = 227 * 1024 - 1024;  // dynamic shared memory: the opt-in limit less the
+                                                // static barriers
 constexpr int kThreads = 320;        // warp 0: TMA, warp 1: MMA, warps 2-9: epilogue
 constexpr int kEpiThreads = 256;
 constexpr uint32_t kTmemCols = 512;  // two 256-column FP32 accumulators
-constexpr int kChunkKB = 60;         // K blocks per accumulator chunk: 60 x 4 = 240 MMAs
+constexpr int kChunkMma = 240;       // MMAs of an accumulator chunk
 
 struct TcParams {
-  int Mpad, Npad, KB;   // padded batch rows per (class, part), padded columns, K blocks of 64
+  int Mpad, KB;         // padded batch rows per (class, part), K blocks of 64
+  int brow[8];          // first row of the class in B's map (64 K entries a row)
   int M;                // valid batch rows
+  int mt;               // batch blocks
   int ncols[8];         // valid columns per class
   int coff[8];          // column offset of the class inside C
+  int tn[8], first[9];  // columns of a tile of the class; the class's first tile / mt
   int ldc;              // row stride of C (floats)
+  int stages, stage_bytes;
   int stall;            // test hook: no loads are issued, and waits give up after kStallPolls
-  int ntn;              // N tiles per class
-  const int* split;     // (8, ntn): 1 = hi+lo split (three K segments), 0 = plain BF16 (one)
+  int ntn;              // row length of split
+  const int* split;     // (8, ntn): 1 = hi+lo split (three products), 0 = plain BF16 (one)
+  int whole;            // tiles below this are one unit each
+  int parts, q;         // units of the others: parts of q chunks
+  int slots;            // slabs of a split tile
+  float* slab;          // [split tile][slot][column][row], 256 x 128 floats each
+  int* count;           // parts of each split tile that have arrived (zero before the launch)
+};
+
+struct BMaps {
+  CUtensorMap m[8];     // per class: its tile's rows, TK (or, interleaved, TKI) of a row
 };
 
 // Poll limit of every wait while the stall hook is on: at most kStallPolls x kSuspendNs (20 ms).
 constexpr long long kStallPolls = 1 << 10;
 
-// Instruction descriptor, kind::f16: D f32, A/B bf16, both K-major, M=128, N=256.
-constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TN >> 3) << 17) | ((uint32_t)(TM >> 4) << 24);
-
-__device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-      " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem_d),
-      "l"(adesc), "l"(bdesc), "r"(kIdesc), "r"(accumulate));
-}
-
-__device__ __forceinline__ void mma_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
-               : "memory");
-}
-
 __device__ __forceinline__ void mbar_arrive_cta(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
+// INTERLEAVED: the order of the products (see above); it takes split tiles only.
+template <bool INTERLEAVED>
 __global__ void __launch_bounds__(kThreads, 1)
-gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, TcParams P,
-               float* __restrict__ C, int* __restrict__ err) {
+gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ BMaps mapB,
+               const __grid_constant__ TcParams P, float* __restrict__ C, int* __restrict__ err) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   // 1024-byte alignment for the swizzled tiles
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  __shared__ __align__(8) uint64_t full_bar[STAGES];
-  __shared__ __align__(8) uint64_t empty_bar[STAGES];
+  __shared__ __align__(8) uint64_t full_bar[kMaxStages];
+  __shared__ __align__(8) uint64_t empty_bar[kMaxStages];
   __shared__ __align__(8) uint64_t acc_full[2], acc_empty[2], drain_bar;
   __shared__ uint32_t tmem_base;
+  __shared__ int last_part;
   __shared__ volatile int abort_flag;
 
-  const int cls = blockIdx.z;
-  // M tiles vary fastest: the CTAs of one basis N-tile run together and read its B slab from
-  // L2 rather than once per M tile from DRAM
-  const int m0 = blockIdx.x * TM, n0 = blockIdx.y * TN;
-  if (n0 >= P.ncols[cls]) return;  // uniform per CTA
+  // this CTA's unit: a tile and the chunks [c0, c1) of its K steps.  M tiles vary fastest, so that
+  // the CTAs of one basis N-tile run together and read its B slab from L2 rather than once per M
+  // tile from DRAM
+  const int unit = blockIdx.x;
+  const bool is_split = unit >= P.whole;
+  const int tile = is_split ? P.whole + (unit - P.whole) / P.parts : unit;
+  const int part = is_split ? (unit - P.whole) % P.parts : 0;
+  const int nt = tile / P.mt;
+  int cls = 0;
+  while (nt >= P.first[cls + 1]) ++cls;
+  const int n = nt - P.first[cls], tn = P.tn[cls];
+  const int m0 = (tile - nt * P.mt) * TM, n0 = n * tn;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // K blocks: the three hi/lo segments, or the (hi, hi) segment alone for a plain BF16 tile
-  const int KB3 = (__ldg(&P.split[cls * P.ntn + blockIdx.y]) ? 3 : 1) * P.KB;
-  const int nchunks = (KB3 + kChunkKB - 1) / kChunkKB;
+  // K steps: the three segments' blocks, or the (hi, hi) segment alone for a plain BF16 tile
+  const int steps = INTERLEAVED ? P.KB * (TK / TKI) : (__ldg(&P.split[cls * P.ntn + n]) ? 3 : 1) * P.KB;
+  constexpr int kSteps = INTERLEAVED ? kChunkMma / (3 * TKI / 16) : kChunkMma / 4;  // of a chunk
+  const int nchunks = (steps + kSteps - 1) / kSteps;
+  const int c0 = part * P.q, c1 = is_split ? min(nchunks, c0 + P.q) : nchunks;
+  if (c0 >= nchunks) return;  // a part past the end of a plain BF16 tile's steps; uniform per CTA
+  const int j0 = c0 * kSteps, j1 = min(steps, c1 * kSteps);
+  const int S = P.stages, b_tile = tn * (INTERLEAVED ? TKI : TK) * 2;
   const long long polls = P.stall ? kStallPolls : kSpinLimit;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < STAGES; ++s) {
+    for (int s = 0; s < S; ++s) {
       mbar_init(&full_bar[s], 1);
       mbar_init(&empty_bar[s], 1);
     }
@@ -134,29 +164,48 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
 
   if (warp == 0 && lane == 0) {
     // ---- TMA producer (the stall hook issues nothing, so the MMA thread's first wait runs out)
-    for (int j = 0; j < KB3 && !abort_flag && !P.stall; ++j) {
-      const int s = j % STAGES;
-      const uint32_t use = j / STAGES;
-      if (j >= STAGES && !mbar_wait_n(&empty_bar[s], (use - 1) & 1, polls)) {
+    int s = 0, seg = INTERLEAVED ? 0 : j0 / P.KB, kb = INTERLEAVED ? j0 : j0 - seg * P.KB;
+    const int ntc = P.first[cls + 1] - P.first[cls], brow = P.brow[cls] + n * P.KB * tn;
+    uint32_t phase = 1;  // of the stage's release before this use (none before the first)
+    for (int j = j0; j < j1 && !abort_flag && !P.stall; ++j) {
+      if (j - j0 >= S && !mbar_wait_n(&empty_bar[s], phase, polls)) {
         atomicCAS(err, 0, 1);
         abort_flag = 1;
         break;
       }
-      const int part = j / P.KB;           // 0: (hi, hi), 1: (lo, hi), 2: (hi, lo)
-      const int kb = j - part * P.KB;
-      const int apart = (part == 1) ? 1 : 0, bpart = (part == 2) ? 1 : 0;
-      uint8_t* sa = smem + s * STAGE_BYTES;
-      mbar_expect_tx(&full_bar[s], STAGE_BYTES);
-      tma_load_2d(sa, &mapA, kb * TK, (cls * 2 + apart) * P.Mpad + m0, &full_bar[s]);
-      tma_load_2d(sa + A_TILE, &mapB, kb * TK, (cls * 2 + bpart) * P.Npad + n0, &full_bar[s]);
+      uint8_t* sa = smem + s * P.stage_bytes;
+      if (INTERLEAVED) {  // A_hi, A_lo, B_hi, B_lo
+        mbar_expect_tx(&full_bar[s], 2 * (AI_TILE + b_tile));
+        const int blk = kb / (TK / TKI), x = (kb % (TK / TKI)) * TKI;
+        for (int h = 0; h < 2; ++h) {
+          tma_load_2d(sa + h * AI_TILE, &mapA, kb * TKI, (cls * 2 + h) * P.Mpad + m0, &full_bar[s]);
+          tma_load_2d(sa + 2 * AI_TILE + h * b_tile, &mapB.m[cls], x, brow + (h * ntc * P.KB + blk) * tn, &full_bar[s]);
+        }
+      } else {
+        // segment 0: (hi, hi), 1: (lo, hi), 2: (hi, lo)
+        const int apart = (seg == 1) ? 1 : 0, bpart = (seg == 2) ? 1 : 0;
+        mbar_expect_tx(&full_bar[s], A_TILE + b_tile);
+        tma_load_2d(sa, &mapA, kb * TK, (cls * 2 + apart) * P.Mpad + m0, &full_bar[s]);
+        tma_load_2d(sa + A_TILE, &mapB.m[cls], 0, brow + (bpart * ntc * P.KB + kb) * tn, &full_bar[s]);
+      }
+      if (++kb == P.KB && !INTERLEAVED) {
+        kb = 0;
+        ++seg;
+      }
+      if (++s == S) {
+        s = 0;
+        phase ^= 1;
+      }
     }
   } else if (warp == 1 && lane == 0) {
-    // ---- MMA issuer: chunk c of kChunkKB K blocks into accumulator c & 1
+    // ---- MMA issuer: this unit's chunk i into accumulator i & 1
+    const uint32_t idesc = idesc_bf16(TM, tn);
     bool ok = true;
-    int issued = 0;
-    for (int c = 0; c < nchunks && ok; ++c) {
-      const int buf = c & 1;
-      if (c >= 2 && !mbar_wait_n(&acc_empty[buf], ((c >> 1) - 1) & 1, polls)) {
+    int issued = 0, s = 0;
+    uint32_t phase = 0;
+    for (int c = c0; c < c1 && ok; ++c) {
+      const int i = c - c0, buf = i & 1;
+      if (i >= 2 && !mbar_wait_n(&acc_empty[buf], ((i >> 1) - 1) & 1, polls)) {
         atomicCAS(err, 0, 4);
         abort_flag = 1;
         ok = false;
@@ -164,46 +213,66 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t d = tmem + (uint32_t)(buf * TN);
-      const int j1 = (c + 1) * kChunkKB < KB3 ? (c + 1) * kChunkKB : KB3;
-      for (int j = c * kChunkKB; j < j1; ++j) {
-        const int s = j % STAGES;
-        const uint32_t use = j / STAGES;
-        if (abort_flag || !mbar_wait_n(&full_bar[s], use & 1, polls)) {
+      const int je = min(j1, (c + 1) * kSteps);
+      for (int j = c * kSteps; j < je; ++j) {
+        if (abort_flag || !mbar_wait_n(&full_bar[s], phase, polls)) {
           atomicCAS(err, 0, 2);
           abort_flag = 1;
           ok = false;
           break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint8_t* sa = smem + s * STAGE_BYTES;
-        const uint64_t ad = smem_desc(sa), bd = smem_desc(sa + A_TILE);
+        const uint8_t* sa = smem + s * P.stage_bytes;
+        const bool fresh = j == c * kSteps;
+        if (INTERLEAVED) {
+          const uint64_t ah = smem_desc64(sa), alo = smem_desc64(sa + AI_TILE), bh = smem_desc64(sa + 2 * AI_TILE),
+                         blo = smem_desc64(sa + 2 * AI_TILE + b_tile);
 #pragma unroll
-        for (int kk = 0; kk < TK / 16; ++kk) {
-          // 16 bf16 = 32 bytes further along K inside the swizzle atom: +2 in the >>4 address field
-          mma_bf16(d, ad + (uint64_t)(kk * 2), bd + (uint64_t)(kk * 2), (j > c * kChunkKB || kk > 0) ? 1u : 0u);
+          for (int kk = 0; kk < TKI / 16; ++kk) {
+            const uint64_t o = (uint64_t)(kk * 2);
+            mma_bf16_id(d, ah + o, bh + o, idesc, (!fresh || kk > 0) ? 1u : 0u);
+            mma_bf16_id(d, alo + o, bh + o, idesc, 1u);
+            mma_bf16_id(d, ah + o, blo + o, idesc, 1u);
+          }
+        } else {
+          const uint64_t ad = smem_desc(sa), bd = smem_desc(sa + A_TILE);
+#pragma unroll
+          for (int kk = 0; kk < TK / 16; ++kk) {
+            // 16 bf16 = 32 bytes further along K inside the swizzle atom: +2 in the >>4 address field
+            mma_bf16_id(d, ad + (uint64_t)(kk * 2), bd + (uint64_t)(kk * 2), idesc, (!fresh || kk > 0) ? 1u : 0u);
+          }
         }
-        mma_commit(&empty_bar[s]);
+        mma_commit_to(&empty_bar[s]);
         ++issued;
+        if (++s == S) {
+          s = 0;
+          phase ^= 1;
+        }
       }
-      if (ok) mma_commit(&acc_full[buf]);
+      if (ok) mma_commit_to(&acc_full[buf]);
     }
     if (!ok && issued > 0) {
       // let the MMAs already issued finish before the tensor memory is freed
-      mma_commit(&drain_bar);
+      mma_commit_to(&drain_bar);
       mbar_wait_n(&drain_bar, 0, polls);
     }
   } else if (warp >= 2) {
     // ---- epilogue: warp w reads TMEM lanes 32*(w%4) .. +31 (rows m0 + that range), columns
     // h*128 .. +127 with h = (w-2)/4, and keeps their running sums over the chunks
     const int q = warp & 3, h = (warp - 2) >> 2;
-    const int row = m0 + q * 32 + lane;
+    const int row = q * 32 + lane;
+    const bool valid = m0 + row < P.M;
+    const int ncol = min(tn, P.ncols[cls] - n0);  // valid columns of the tile
+    // slab column 0 of this thread's row and half; chunk c of a part after the first goes to slot
+    // c - q, or the whole part to slot part - 1
+    float* slab = P.slab + ((int64_t)(tile - P.whole) * P.slots * TN + h * (TN / 2)) * TM + row;
     float acc[TN / 2];
 #pragma unroll
     for (int t = 0; t < TN / 2; ++t) acc[t] = 0.f;
     bool done = true;
-    for (int c = 0; c < nchunks; ++c) {
-      const int buf = c & 1;
-      if (abort_flag || !mbar_wait_n(&acc_full[buf], (c >> 1) & 1, polls)) {
+    for (int c = c0; c < c1; ++c) {
+      const int i = c - c0, buf = i & 1;
+      if (abort_flag || !mbar_wait_n(&acc_full[buf], (i >> 1) & 1, polls)) {
         atomicCAS(err, 0, 3);
         abort_flag = 1;
         done = false;
@@ -211,6 +280,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * TN + h * (TN / 2));
+      const bool to_slab = !INTERLEAVED && part > 0;
+      float* out = slab + (int64_t)(c - P.q) * TN * TM;
 #pragma unroll
       for (int cb = 0; cb < TN / 2; cb += 32) {
         uint32_t v[32];
@@ -224,19 +295,70 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
               "=r"(v[30]), "=r"(v[31])
             : "r"(taddr + (uint32_t)cb));
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        if (to_slab) {
+          if (valid) {
 #pragma unroll
-        for (int t = 0; t < 32; ++t) acc[cb + t] += __uint_as_float(v[t]);
+            for (int t = 0; t < 32; ++t)
+              if (h * (TN / 2) + cb + t < ncol) out[(cb + t) * TM] = __uint_as_float(v[t]);
+          }
+        } else {
+#pragma unroll
+          for (int t = 0; t < 32; ++t) acc[cb + t] += __uint_as_float(v[t]);
+        }
       }
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       mbar_arrive_cta(&acc_empty[buf]);
     }
-    if (done && row < P.M) {
-      float* crow = C + (int64_t)row * P.ldc + P.coff[cls];
-      const int nc = P.ncols[cls];
-      const int nb = n0 + h * (TN / 2);
+    float* crow = C + (int64_t)(m0 + row) * P.ldc + P.coff[cls] + n0 + h * (TN / 2);
+    if (done && valid) {
+      if (part == 0) {
 #pragma unroll
-      for (int t = 0; t < TN / 2; ++t)
-        if (nb + t < nc) crow[nb + t] = acc[t];
+        for (int t = 0; t < TN / 2; ++t)
+          if (h * (TN / 2) + t < ncol) crow[t] = acc[t];
+      } else if (INTERLEAVED) {
+        float* out = slab + (int64_t)(part - 1) * TN * TM;
+#pragma unroll
+        for (int t = 0; t < TN / 2; ++t)
+          if (h * (TN / 2) + t < ncol) out[t * TM] = acc[t];
+      }
+    }
+    if (is_split && P.parts > 1) {
+      // the part that arrives last adds the slabs to C, in order (a part that gave up does not
+      // arrive: the call has failed then)
+      __threadfence();
+      asm volatile("bar.sync 1, %0;" ::"n"(kEpiThreads) : "memory");
+      if (threadIdx.x == 64) {
+        const int total = (nchunks + P.q - 1) / P.q;
+        last_part = !abort_flag && atomicAdd(&P.count[tile - P.whole], 1) == total - 1;
+      }
+      asm volatile("bar.sync 1, %0;" ::"n"(kEpiThreads) : "memory");
+      if (last_part) {
+        __threadfence();
+        const int slots = INTERLEAVED ? (nchunks + P.q - 1) / P.q - 1 : nchunks - P.q;
+        const int rows = min(TM, P.M - m0), total = rows * ncol;
+        const float* slab0 = P.slab + (int64_t)(tile - P.whole) * P.slots * TN * TM;
+        float* c0p = C + (int64_t)m0 * P.ldc + P.coff[cls] + n0;
+        constexpr int U = 4;  // elements of a thread in flight
+        for (int e = (int)threadIdx.x - 64; e < total; e += U * kEpiThreads) {
+          float v[U];
+          float* at[U];
+          const float* from[U];
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            const int i = min(e + u * kEpiThreads, total - 1), col = i / rows, r = i - col * rows;
+            at[u] = c0p + (int64_t)r * P.ldc + col;
+            from[u] = slab0 + col * TM + r;
+            v[u] = __ldcg(at[u]);
+          }
+#pragma unroll 4
+          for (int k = 0; k < slots; ++k)
+#pragma unroll
+            for (int u = 0; u < U; ++u) v[u] += __ldcg(from[u] + (int64_t)k * TN * TM);
+#pragma unroll
+          for (int u = 0; u < U; ++u)
+            if (e + u * kEpiThreads < total) *at[u] = v[u];
+        }
+      }
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -250,9 +372,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
 // ---------------------------------------------------------------- operand preparation
 // Folded channels, split into bf16 hi/lo: Aall[((cls*2 + part) * Mpad + b) * Kpad + rep].
 __global__ void fold_split_kernel(const float* __restrict__ vol, int64_t vol_stride, int B, int n_rep, int Mpad,
-                                  int Kpad, const int* __restrict__ rep_img, __nv_bfloat16* __restrict__ A) {
+                                  int Kpad, const int* __restrict__ rep_img, __nv_bfloat16* __restrict__ A,
+                                  int* __restrict__ count, int n_count) {
   const int rep = blockIdx.x * blockDim.x + threadIdx.x;
   const int b = blockIdx.y;
+  if (blockIdx.x == 0 && b == 0)  // the arrival counts of the GEMM that follows
+    for (int i = threadIdx.x; i < n_count; i += blockDim.x) count[i] = 0;
   if (rep >= Kpad || b >= B) return;
   float f[8];
 #pragma unroll
@@ -278,8 +403,8 @@ __global__ void fold_split_kernel(const float* __restrict__ vol, int64_t vol_str
   }
 }
 
-// Basis (K x n_p, row-major FP32 per class) -> Ball[((cls*2 + part) * Npad + n) * Kpad + k], K-major bf16.
-__global__ void basis_split_kernel(const float* __restrict__ basis, int n_rep, int ncls, int cls, int Npad, int Kpad,
+// Basis (K x n_p, row-major FP32 per class) -> the class's tiles [part][n / tn][k / 64][n % tn][k % 64] at Bm.
+__global__ void basis_split_kernel(const float* __restrict__ basis, int n_rep, int ncls, int nt, int tn, int Kpad,
                                    __nv_bfloat16* __restrict__ Bm) {
   __shared__ float tile[32][33];
   const int k0 = blockIdx.x * 32, n0 = blockIdx.y * 32;
@@ -288,14 +413,16 @@ __global__ void basis_split_kernel(const float* __restrict__ basis, int n_rep, i
     tile[i][threadIdx.x] = (k < n_rep && n < ncls) ? basis[(int64_t)k * ncls + n] : 0.f;
   }
   __syncthreads();
+  const int KB = Kpad / TK;
   for (int i = threadIdx.y; i < 32; i += blockDim.y) {
     const int n = n0 + i, k = k0 + threadIdx.x;
-    if (n >= Npad || k >= Kpad) continue;
+    if (n >= nt * tn || k >= Kpad) continue;
     const float v = tile[threadIdx.x][i];
     uint32_t hi, lo;
     split_bf16(v, hi, lo);
-    Bm[((int64_t)(cls * 2 + 0) * Npad + n) * Kpad + k] = __ushort_as_bfloat16((unsigned short)hi);
-    Bm[((int64_t)(cls * 2 + 1) * Npad + n) * Kpad + k] = __ushort_as_bfloat16((unsigned short)lo);
+    const int64_t at = (((int64_t)(n / tn) * KB + k / TK) * tn + n % tn) * TK + k % TK;
+    Bm[at] = __ushort_as_bfloat16((unsigned short)hi);
+    Bm[(int64_t)nt * KB * tn * TK + at] = __ushort_as_bfloat16((unsigned short)lo);
   }
 }
 
@@ -303,7 +430,7 @@ typedef CUresult (*EncodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, v
                                 const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                 CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
-int make_map(CUtensorMap* map, void* base, uint64_t inner, uint64_t rows, uint32_t box_rows) {
+int make_map(CUtensorMap* map, void* base, uint64_t inner, uint64_t rows, uint32_t box_rows, uint32_t box_k) {
   static EncodeTiled fn = nullptr;
   if (!fn) {
     cudaDriverEntryPointQueryResult q;
@@ -315,12 +442,64 @@ int make_map(CUtensorMap* map, void* base, uint64_t inner, uint64_t rows, uint32
   }
   const cuuint64_t dims[2] = {inner, rows};
   const cuuint64_t strides[1] = {inner * 2};
-  const cuuint32_t box[2] = {(cuuint32_t)TK, box_rows};
+  const cuuint32_t box[2] = {box_k, box_rows};
   const cuuint32_t estr[2] = {1, 1};
   const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, dims, strides, box, estr,
-                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                        CU_TENSOR_MAP_INTERLEAVE_NONE,
+                        box_k == TKI ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? MTB_OK : MTB_ERR_CUDA;
+}
+
+constexpr int kSMs = 148;
+constexpr size_t kSlabCap = (size_t)128 << 20;  // bytes of slabs a plan may take
+
+// How a GEMM of mt batch blocks is cut into units.
+struct GemmPlan {
+  bool interleaved;
+  int tiles, whole, parts, q, slots, units;
+};
+
+// Tiles beyond the whole rounds of the SMs are cut into parts of q chunks; q minimises the rounds
+// times their length (a quarter chunk for a unit's start and end) plus the slabs' way to memory and
+// back (about 18 us a chunk and 6.5 GB/ms).  One batch block of 48^3 (16 tiles of 5 chunks) runs as
+// 80 units instead of 16, 100 subtomograms of 96^3 (117 tiles of 40) as 585 instead of 117.
+// The interleaved order is for a basis larger than L2 (126 MB); see the top.
+GemmPlan gemm_plan(const FleTc* t, int mt) {
+  GemmPlan p;
+  const int KB = t->Kpad / TK;
+  int nt = 0;
+  size_t cols = 0;
+  for (int k = 0; k < 8; ++k) {
+    nt += t->nt[k];
+    cols += t->ncols[k];
+  }
+  const bool all_split = t->n_split_tiles == t->n_tiles;
+  p.interleaved = all_split && cols * t->Kpad * 4 > ((size_t)126 << 20);
+  const int nchunks = (KB * 12 + kChunkMma - 1) / kChunkMma;
+  p.tiles = nt * mt;
+  p.whole = p.tiles / kSMs * kSMs;
+  const int rest = p.tiles - p.whole;
+  p.parts = 1;
+  p.q = nchunks;
+  p.slots = 0;
+  double best = 1e30;
+  for (int q = nchunks; q >= 1 && rest > 0; --q) {
+    const int parts = (nchunks + q - 1) / q;
+    const int slots = parts == 1 ? 0 : (p.interleaved ? parts - 1 : nchunks - q);
+    const size_t bytes = (size_t)rest * slots * TN * TM * sizeof(float);
+    if (bytes > kSlabCap) continue;
+    const int rounds = (rest * parts + kSMs - 1) / kSMs;
+    const double cost = rounds * (q + 0.25) + 2.0 * bytes / 6.5e9 / 0.018;
+    if (cost < best - 1e-9) {
+      best = cost;
+      p.parts = parts;
+      p.q = q;
+      p.slots = slots;
+    }
+  }
+  p.units = p.whole + rest * p.parts;
+  return p;
 }
 
 }  // namespace
@@ -338,19 +517,29 @@ int fle_tc_prepare(FleTc* t, float* const* basis, const int* class_cols, const i
   t->Kpad = (n_rep + TK - 1) / TK * TK;
   int maxc = 0;
   for (int k = 0; k < 8; ++k) maxc = class_cols[k] > maxc ? class_cols[k] : maxc;
-  t->Npad = (maxc + TN - 1) / TN * TN;
   t->n_rep = n_rep;
   t->n_cols = n_cols;
   for (int k = 0; k < 8; ++k) {
     t->ncols[k] = class_cols[k];
     t->coff[k] = class_off[k];
+    // the class's columns cut evenly into the fewest tiles, in steps of 16 (with a degree
+    // schedule, which is by tiles of 256, they stay 256)
+    t->nt[k] = (class_cols[k] + TN - 1) / TN;
+    t->tn[k] = TN;
+    if (t->nt[k] && split_degree < 0) t->tn[k] = ((class_cols[k] + t->nt[k] - 1) / t->nt[k] + 15) / 16 * 16;
   }
-  const size_t asz = (size_t)16 * t->Mpad * t->Kpad, bsz = (size_t)16 * t->Npad * t->Kpad;
+  int64_t rows = 0;  // of 64 K entries
+  for (int k = 0; k < 8; ++k) {
+    t->brow[k] = (int)rows;
+    rows += (int64_t)2 * t->nt[k] * (t->Kpad / TK) * t->tn[k];
+  }
+  if (rows > 0x7fffffff) return MTB_ERR_ARG;  // TMA coordinates
+  const size_t asz = (size_t)16 * t->Mpad * t->Kpad, bsz = (size_t)rows * TK;
   if (cudaMalloc(&t->A, asz * 2) != cudaSuccess) return MTB_ERR_OOM;
   if (cudaMalloc(&t->B, bsz * 2) != cudaSuccess) return MTB_ERR_OOM;
   if (cudaMalloc(&t->err, sizeof(int)) != cudaSuccess) return MTB_ERR_OOM;
   // which tiles take the split: those holding a column of degree above split_degree
-  t->ntn = t->Npad / TN;
+  t->ntn = (maxc + TN - 1) / TN;
   {
     std::vector<int> flags((size_t)8 * t->ntn, 1);
     for (int k = 0; k < 8; ++k)
@@ -372,15 +561,31 @@ int fle_tc_prepare(FleTc* t, float* const* basis, const int* class_cols, const i
     return MTB_ERR_CUDA;
   for (int k = 0; k < 8; ++k) {
     if (!class_cols[k]) continue;
-    dim3 g((t->Kpad + 31) / 32, (t->Npad + 31) / 32);
-    basis_split_kernel<<<g, dim3(32, 8)>>>(basis[k], n_rep, class_cols[k], k, t->Npad, t->Kpad,
-                                           reinterpret_cast<__nv_bfloat16*>(t->B));
+    dim3 g((t->Kpad + 31) / 32, (t->nt[k] * t->tn[k] + 31) / 32);
+    basis_split_kernel<<<g, dim3(32, 8)>>>(basis[k], n_rep, class_cols[k], t->nt[k], t->tn[k], t->Kpad,
+                                           reinterpret_cast<__nv_bfloat16*>(t->B) + (int64_t)t->brow[k] * TK);
     if (cudaGetLastError() != cudaSuccess) return MTB_ERR_CUDA;
   }
   if (cudaDeviceSynchronize() != cudaSuccess) return MTB_ERR_CUDA;
-  int rc = make_map(reinterpret_cast<CUtensorMap*>(t->mapA), t->A, (uint64_t)t->Kpad, (uint64_t)16 * t->Mpad, TM);
-  if (!rc) rc = make_map(reinterpret_cast<CUtensorMap*>(t->mapB), t->B, (uint64_t)t->Kpad, (uint64_t)16 * t->Npad, TN);
-  return rc;
+  int rc = MTB_OK;
+  for (int i = 0; i < 2 && !rc; ++i) {  // stages of TK, of TKI
+    const uint32_t k = i ? TKI : TK;
+    rc = make_map(reinterpret_cast<CUtensorMap*>(t->mapA[i]), t->A, (uint64_t)t->Kpad, (uint64_t)16 * t->Mpad, TM, k);
+    for (int c = 0; c < 8 && !rc; ++c)
+      rc = make_map(reinterpret_cast<CUtensorMap*>(t->mapB[i][c]), t->B, TK, (uint64_t)rows, (uint32_t)t->tn[c], k);
+  }
+  if (rc) return rc;
+  // slabs and arrival counts of every batch up to max_batch
+  size_t slab = 0;
+  for (int mt = 1; mt <= t->Mpad / TM; ++mt) {
+    const GemmPlan p = gemm_plan(t, mt);
+    const size_t n = (size_t)(p.tiles - p.whole) * p.slots * TN * TM * sizeof(float);
+    slab = n > slab ? n : slab;
+    if (p.parts > 1 && p.tiles - p.whole > t->n_count) t->n_count = p.tiles - p.whole;
+  }
+  if (slab && cudaMalloc(&t->slab, slab) != cudaSuccess) return MTB_ERR_OOM;
+  if (t->n_count && cudaMalloc(&t->count, t->n_count * sizeof(int)) != cudaSuccess) return MTB_ERR_OOM;
+  return MTB_OK;
 }
 
 void fle_tc_release(FleTc* t) {
@@ -388,6 +593,8 @@ void fle_tc_release(FleTc* t) {
   if (t->B) cudaFree(t->B);
   if (t->err) cudaFree(t->err);
   if (t->split) cudaFree(t->split);
+  if (t->slab) cudaFree(t->slab);
+  if (t->count) cudaFree(t->count);
   memset(t, 0, sizeof(*t));
 }
 
@@ -396,28 +603,45 @@ int fle_tc_forward(FleTc* t, const float* vol, int64_t vol_stride, int B, const 
   dim3 fg((t->Kpad + 255) / 256, B);
   mtb_prof_begin(st);
   fold_split_kernel<<<fg, 256, 0, st>>>(vol, vol_stride, B, t->n_rep, t->Mpad, t->Kpad, rep_img,
-                                        reinterpret_cast<__nv_bfloat16*>(t->A));
+                                        reinterpret_cast<__nv_bfloat16*>(t->A), t->count, t->n_count);
   mtb_prof_end(st, "fold_split_kernel");
   MTB_LAUNCH_CHECK();
   TcParams P;
   P.Mpad = t->Mpad;
-  P.Npad = t->Npad;
   P.KB = t->Kpad / TK;
   P.M = B;
+  P.mt = (B + TM - 1) / TM;
+  const GemmPlan plan = gemm_plan(t, P.mt);
+  int tn_max = 16;
+  P.first[0] = 0;
   for (int k = 0; k < 8; ++k) {
     P.ncols[k] = t->ncols[k];
     P.coff[k] = t->coff[k];
+    P.tn[k] = t->tn[k];
+    P.brow[k] = t->brow[k];
+    P.first[k + 1] = P.first[k] + t->nt[k];
+    if (t->nt[k] && t->tn[k] > tn_max) tn_max = t->tn[k];
   }
   P.ldc = t->n_cols;
+  // stages on 1024-byte boundaries (a B tile of 16 rows is 2 KB)
+  P.stage_bytes = A_TILE + tn_max * TK * 2;  // the same for both orders
+  P.stages = (int)((kSmemCap - 1024) / P.stage_bytes);
+  if (P.stages > kMaxStages) P.stages = kMaxStages;
   P.stall = t->stall;
   P.ntn = t->ntn;
   P.split = t->split;
-  const size_t smem = (size_t)STAGES * STAGE_BYTES + 1024;
-  MTB_CUDA_TRY(cudaFuncSetAttribute(gemm_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  dim3 gg((B + TM - 1) / TM, t->Npad / TN, 8);
+  P.whole = plan.whole;
+  P.parts = plan.parts;
+  P.q = plan.q;
+  P.slots = plan.slots;
+  P.slab = t->slab;
+  P.count = t->count;
+  const size_t smem = (size_t)P.stages * P.stage_bytes + 1024;
+  const auto kernel = plan.interleaved ? gemm_tc_kernel<true> : gemm_tc_kernel<false>;
+  MTB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   mtb_prof_begin(st);
-  gemm_tc_kernel<<<gg, kThreads, smem, st>>>(*reinterpret_cast<const CUtensorMap*>(t->mapA),
-                                             *reinterpret_cast<const CUtensorMap*>(t->mapB), P, C, t->err);
+  kernel<<<plan.units, kThreads, smem, st>>>(*reinterpret_cast<const CUtensorMap*>(t->mapA[plan.interleaved]),
+                                             *reinterpret_cast<const BMaps*>(t->mapB[plan.interleaved]), P, C, t->err);
   mtb_prof_end(st, "gemm_tc_kernel");
   MTB_LAUNCH_CHECK();
   return MTB_OK;

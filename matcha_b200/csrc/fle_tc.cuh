@@ -6,17 +6,24 @@
 #include <vector>
 
 struct FleTc {
-  alignas(64) unsigned char mapA[128];  // CUtensorMap of the folded channels (bf16 hi/lo)
-  alignas(64) unsigned char mapB[128];  // CUtensorMap of the basis (bf16 hi/lo, K-major)
-  int Mpad, Npad, Kpad, n_rep, n_cols;
+  // CUtensorMaps of the folded channels and, per class, of the basis (bf16 hi/lo, K-major), for
+  // stages of 64 and of 32 along K
+  alignas(64) unsigned char mapA[2][128];
+  alignas(64) unsigned char mapB[2][8][128];
+  int Mpad, Kpad, n_rep, n_cols;
   int ncols[8], coff[8];
+  int nt[8], tn[8];  // per class: column tiles and their width
+  int brow[8];       // per class: first row of its tiles in B (64 K entries a row)
   void* A;   // (8 classes x 2 parts x Mpad, Kpad) bf16
-  void* B;   // (8 classes x 2 parts x Npad, Kpad) bf16
+  void* B;   // [class][hi, lo][column tile][K block][column][64] bf16
   int* err;  // nonzero after a bounded wait ran out
   int stall; // test hook (mtb_fle_inject_stall): the producer issues no loads, waits give up early
-  int ntn;   // 256-column tiles per class (Npad / 256)
+  int ntn;   // column tiles of the largest class
   int* split;  // (8, ntn): 1 where the tile takes the hi+lo split (three MMAs per K step), 0 where
                // its columns are all of degree <= split_degree (plain BF16, one MMA)
+  float* slab;  // partial sums of the tiles cut along K
+  int* count;   // their parts that have arrived
+  int n_count;
   int n_split_tiles, n_tiles;  // how many of the valid tiles take the split, of how many
 };
 

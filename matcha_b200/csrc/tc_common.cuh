@@ -68,6 +68,17 @@ __device__ __forceinline__ uint64_t smem_desc(const void* p) {
   return d;
 }
 
+// The same for 64-byte rows (32 bf16): 64-byte swizzle, 8-row groups 512 B apart.
+__device__ __forceinline__ uint64_t smem_desc64(const void* p) {
+  const uint64_t addr = smem_u32(p);
+  uint64_t d = 0;
+  d |= (addr >> 4) & 0x3FFFull;
+  d |= (uint64_t)1 << 16;
+  d |= (uint64_t)(512 >> 4) << 32;
+  d |= (uint64_t)1 << 46;
+  d |= (uint64_t)4 << 61;                 // SWIZZLE_64B
+  return d;
+}
 
 // Instruction descriptor of tcgen05.mma kind::f16: D f32, A and B bf16, both K-major.
 __host__ __device__ constexpr uint32_t idesc_bf16(int M, int N) {
