@@ -15,6 +15,7 @@
 // and the adjoint becomes 8 independent GEMMs of 1/8 the depth and 1/8 the width:
 // 1/8 of the dense work, still exact.  Coefficients with m < 0 follow from
 // a_{l,k,-m} = (-1)^m conj(a_{l,k,m}) for real volumes.
+#include <cooperative_groups.h>
 #include <math.h>
 #include <string.h>
 #include <algorithm>
@@ -183,32 +184,58 @@ gemm_fp32_kernel(const float* __restrict__ A, int64_t a_stride_class, int M, int
 }
 
 // ------------------------------------------------------------------ expand + norms
-// a[b][i] = s_re * C[b][col_re[i]] + i * s_im * C[b][col_im[i]]  (col_im < 0 -> 0)
-__global__ void expand_kernel(const float* __restrict__ C, int64_t c_ld, int B, int ne,
-                              const int* __restrict__ col_re, const int* __restrict__ col_im,
-                              const signed char* __restrict__ s_re, const signed char* __restrict__ s_im,
-                              float2* __restrict__ out, int64_t out_stride, float* __restrict__ norms) {
-  const int b = blockIdx.x;
-  if (b >= B) return;
+// a[b][i] = +-C[b][re_i] +- i C[b][im_i]: cols[i] holds the two columns, each shifted left by one
+// with the sign in bit 0 (-1: no imaginary part).  The work is a gather of a row that L1 holds, so
+// latency sets the time: a cluster of CTAs shares a subtomogram's coefficients, a thread has four
+// in flight, and the cluster's sums of squares meet through distributed shared memory in order.
+// 100 subtomograms of 96^3 18 us, before 111 us; one of 48^3 9 us, before 21 us (one CTA each).
+constexpr int kET = 256;
+
+__device__ __forceinline__ float signed_at(const float* c, int code) {
+  const float v = code >= 0 ? __ldg(c + (code >> 1)) : 0.f;
+  return (code & 1) && code >= 0 ? -v : v;
+}
+
+__global__ void __launch_bounds__(kET)
+expand_kernel(const float* __restrict__ C, int64_t c_ld, int ne, const int2* __restrict__ cols,
+              float2* __restrict__ out, int64_t out_stride, float* __restrict__ norms) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cluster = cg::this_cluster();
+  const int rank = (int)cluster.block_rank(), parts = (int)cluster.num_blocks(), b = blockIdx.y;
   const float* c = C + (int64_t)b * c_ld;
+  float2* o = out + (int64_t)b * out_stride;
   float ss = 0.f;
-  for (int i = threadIdx.x; i < ne; i += blockDim.x) {
-    const float re = s_re[i] * c[col_re[i]];
-    const float im = col_im[i] >= 0 ? s_im[i] * c[col_im[i]] : 0.f;
-    out[(int64_t)b * out_stride + i] = make_float2(re, im);
-    ss += re * re + im * im;
-  }
-  if (norms) {
-    __shared__ float red[32];
-    ss = warp_sum(ss);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-      float v = threadIdx.x < (blockDim.x >> 5) ? red[threadIdx.x] : 0.f;
-      v = warp_sum(v);
-      if (threadIdx.x == 0) norms[b] = sqrtf(v);
+  const int step = parts * kET;
+  for (int i0 = rank * kET + threadIdx.x; i0 < ne; i0 += 4 * step) {
+    int2 k[4];
+    float2 v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) k[u] = i0 + u * step < ne ? __ldg(&cols[i0 + u * step]) : make_int2(-1, -1);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) v[u] = make_float2(signed_at(c, k[u].x), signed_at(c, k[u].y));
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      if (i0 + u * step < ne) o[i0 + u * step] = v[u];
+      ss += v[u].x * v[u].x + v[u].y * v[u].y;
     }
   }
+  if (!norms) return;  // the same for the whole cluster
+  __shared__ float red[kET / 32], total;
+  ss = warp_sum(ss);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    float s = 0.f;
+    for (int w = 0; w < kET / 32; ++w) s += red[w];
+    total = s;
+  }
+  cluster.sync();
+  if (rank == 0 && threadIdx.x == 0) {
+    float s = 0.f;
+    for (int q = 0; q < parts; ++q) s += cluster.map_shared_rank(&total, q)[0];
+    norms[b] = sqrtf(s);
+  }
+  cluster.sync();  // no CTA leaves while its sum is read
 }
 
 // ------------------------------------------------------------------ sigma
@@ -290,10 +317,7 @@ struct mtb_fle {
   int* d_class_cols;
   int* d_class_off;
   int* rep_img;
-  int* col_re;
-  int* col_im;
-  signed char* s_re;
-  signed char* s_im;
+  int2* cols;    // per coefficient: the columns of its parts with their signs (expand_kernel)
   float* A;      // (8, max_batch, n_rep) folded channels
   float* C;      // (max_batch, n_cols) real coefficients, class blocks side by side
   int* kpad;
@@ -358,12 +382,13 @@ extern "C" int mtb_fle_create(const mtb_fle_config* cfg, mtb_fle** out) {
   // global column index of each (class, pos): class_off + pos
   std::vector<int> gcol(nc);
   for (int c = 0; c < nc; ++c) gcol[c] = h->class_off[cfg->col_class[c]] + pos[c];
-  std::vector<int> cre(cfg->ne), cim(cfg->ne);
+  std::vector<int2> cols(cfg->ne);
+  if (nc > (1 << 30)) return fail(MTB_ERR_ARG);
   for (int i = 0; i < cfg->ne; ++i) {
     const int r = cfg->coef_col_re[i], m = cfg->coef_col_im[i];
     if (r < 0 || r >= nc || m >= nc) return fail(MTB_ERR_ARG);
-    cre[i] = gcol[r];
-    cim[i] = m >= 0 ? gcol[m] : -1;
+    cols[i].x = 2 * gcol[r] + (cfg->coef_sign_re[i] < 0);
+    cols[i].y = m >= 0 ? 2 * gcol[m] + (cfg->coef_sign_im[i] < 0) : -1;
   }
   // sigma gather table offsets
   std::vector<int> koff(L + 1);
@@ -386,10 +411,7 @@ extern "C" int mtb_fle_create(const mtb_fle_config* cfg, mtb_fle** out) {
   if (!rc) rc = upload(&h->d_class_cols, h->class_cols, kClasses);
   if (!rc) rc = upload(&h->d_class_off, h->class_off, kClasses);
   if (!rc) rc = upload(&h->rep_img, cfg->rep_img, (size_t)nr * 8);
-  if (!rc) rc = upload(&h->col_re, cre.data(), cre.size());
-  if (!rc) rc = upload(&h->col_im, cim.data(), cim.size());
-  if (!rc) rc = upload(&h->s_re, cfg->coef_sign_re, (size_t)cfg->ne);
-  if (!rc) rc = upload(&h->s_im, cfg->coef_sign_im, (size_t)cfg->ne);
+  if (!rc) rc = upload(&h->cols, cols.data(), cols.size());
   if (!rc) rc = upload(&h->kpad, cfg->kpad, (size_t)L + 1);
   if (!rc) rc = upload(&h->koff, koff.data(), koff.size());
   if (!rc) rc = upload(&h->kidx, cfg->kidx, (size_t)kt);
@@ -454,8 +476,7 @@ extern "C" void mtb_fle_destroy(mtb_fle* h) {
   if (!h) return;
   for (int k = 0; k < kClasses; ++k) if (h->basis[k]) cudaFree(h->basis[k]);
   fle_tc_release(&h->tc);
-  void* ptrs[] = {h->d_basis, h->d_class_cols, h->d_class_off, h->rep_img, h->col_re, h->col_im, h->s_re, h->s_im,
-                  h->A, h->C, h->kpad, h->koff, h->kidx};
+  void* ptrs[] = {h->d_basis, h->d_class_cols, h->d_class_off, h->rep_img, h->cols, h->A, h->C, h->kpad, h->koff, h->kidx};
   for (void* p : ptrs) if (p) cudaFree(p);
   delete[] h->kpad_host;
   delete h;
@@ -491,8 +512,14 @@ extern "C" int mtb_fle_forward(mtb_fle* h, const float* vol, int B, float* coeff
     MTB_LAUNCH_CHECK();
   }
   mtb_prof_begin(st);
-  expand_kernel<<<B, 256, 0, st>>>(h->C, h->cfg.n_cols, B, h->cfg.ne, h->col_re, h->col_im, h->s_re, h->s_im,
-                                   reinterpret_cast<float2*>(coeffs), coeff_stride, norms);
+  const int parts = cluster_size(B, 8);
+  for (int b0 = 0; b0 < B; b0 += 65535) {  // the grid's y limit
+    const int n = B - b0 < 65535 ? B - b0 : 65535;
+    MTB_CUDA_TRY(launch_clusters(expand_kernel, dim3(parts, n), kET, 0, parts, st,
+                                 (const float*)h->C + (int64_t)b0 * h->cfg.n_cols, (int64_t)h->cfg.n_cols, h->cfg.ne,
+                                 (const int2*)h->cols, reinterpret_cast<float2*>(coeffs) + b0 * coeff_stride,
+                                 coeff_stride, norms ? norms + b0 : nullptr));
+  }
   mtb_prof_end(st, "expand_kernel");
   MTB_LAUNCH_CHECK();
   return MTB_OK;
