@@ -119,6 +119,15 @@ int mtb_score_backward(const float* sigma, int64_t sigma_stride, int B, int L, c
                        const float* gamma, const float* weight, float* grad_sigma, int64_t grad_stride,
                        double* grad_body, mtb_stream_t stream);
 
+/* The rotations of a batch around base Euler angles, FP64 on the device (no counterpart in the
+ * reference): alpha, beta, gamma (B,) float32 of Rz(a) Ry(b) Rz(g) exp([omega]x), and the gradient
+ * with respect to omega of a function whose body-frame gradient at that rotation is grad_body,
+ * Jr(omega)^T grad_body (Jr the right Jacobian).  omega, base, grad_body, grad_omega: (B, 3). */
+int mtb_rotation_angles(const double* omega, const double* base, int B, float* alpha, float* beta, float* gamma,
+                        mtb_stream_t stream);
+int mtb_rotation_gradient(const double* omega, const double* grad_body, int B, double* grad_omega,
+                          mtb_stream_t stream);
+
 /* Allocation-free orientation search.  No counterpart in the reference: it is
  * mtb_search_orientations for callers that must not allocate device memory -- a host
  * program that hands all device memory to its own allocator or runs under a fixed

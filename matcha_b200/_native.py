@@ -94,6 +94,8 @@ SIGNATURES = {
     "mtb_fle_split_tiles": (_I, [_P, ctypes.POINTER(_I), ctypes.POINTER(_I)]),
     "mtb_sigma_backward_template": (_I, [_P, _P, _I64, _P, _I64, _I, _I, _P, _P]),
     "mtb_score_backward": (_I, [_P, _I64, _I, _I, _P, _P, _P, _P, _P, _I64, _P, _P]),
+    "mtb_rotation_angles": (_I, [_P, _P, _I, _P, _P, _P, _P]),
+    "mtb_rotation_gradient": (_I, [_P, _P, _I, _P, _P]),
     "mtb_shift_create": (_I, [ctypes.POINTER(MtbShiftConfig), ctypes.POINTER(_P)]),
     "mtb_shift_destroy": (None, [_P]),
     "mtb_shift_set_reference": (_I, [_P, _P, _P]),

@@ -29,6 +29,7 @@ from __future__ import annotations
 import torch
 
 from . import _native as nat
+from .core.wigner_index import dsize
 
 
 def _hat(w):
@@ -105,12 +106,22 @@ class RotationScore(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, omega, sigma, base_angles, matcher, L):
-        w = omega.detach().to(torch.float64)
-        base = base_angles.to(device=w.device, dtype=torch.float64)
-        R = zyz_matrix(base[:, 0], base[:, 1], base[:, 2]) @ so3_exp(w)
-        a, b, g = (_f32(x) for x in zyz_angles(R))
+        w = omega.detach().to(torch.float64).contiguous()
         sig = sigma.detach().contiguous()
-        f, _, _ = matcher.score_derivatives(sig, a, b, g, L)
+        B = w.shape[0]
+        base = base_angles.to(device=w.device, dtype=torch.float64)
+        if w.device == sig.device and sig.is_cuda and w.shape == base.shape == (B, 3):
+            ang = torch.empty((3, B), device=w.device, dtype=torch.float32)
+            base = base.contiguous()
+            with torch.cuda.device(w.device):
+                nat.check(nat.load().mtb_rotation_angles(nat.ptr(w), nat.ptr(base), B, nat.ptr(ang[0]),
+                                                         nat.ptr(ang[1]), nat.ptr(ang[2]),
+                                                         nat.stream_ptr(w.device)), "mtb_rotation_angles")
+            a, b, g = ang.unbind(0)
+        else:
+            R = zyz_matrix(base[:, 0], base[:, 1], base[:, 2]) @ so3_exp(w)
+            a, b, g = (_f32(x) for x in zyz_angles(R))
+        f = matcher.score_and_derivatives(sig, a, b, g, L)[:, 0]
         ctx.save_for_backward(w, sig, a, b, g)
         ctx.L = int(L)
         return f.to(torch.float64)
@@ -121,7 +132,9 @@ class RotationScore(torch.autograd.Function):
         B, L = sig.shape[0], ctx.L
         weight = _f32(grad_out)
         need_sigma = ctx.needs_input_grad[1]
-        grad_sigma = torch.zeros_like(sig) if need_sigma else None
+        grad_sigma = None
+        if need_sigma:  # the kernel writes the degrees <= L: what lies past them is zero
+            grad_sigma = torch.empty_like(sig) if sig.shape[1] == dsize(L) else torch.zeros_like(sig)
         grad_body = torch.empty((B, 3), device=sig.device, dtype=torch.float64)
         lib = nat.load()
         with torch.cuda.device(sig.device):
@@ -129,6 +142,11 @@ class RotationScore(torch.autograd.Function):
                                              nat.ptr(weight), nat.ptr(grad_sigma),
                                              grad_sigma.stride(0) if need_sigma else 0, nat.ptr(grad_body),
                                              nat.stream_ptr(sig.device)), "mtb_score_backward")
+            if w.device == sig.device and w.shape == (B, 3):
+                grad_omega = torch.empty_like(w)
+                nat.check(lib.mtb_rotation_gradient(nat.ptr(w), nat.ptr(grad_body), B, nat.ptr(grad_omega),
+                                                    nat.stream_ptr(sig.device)), "mtb_rotation_gradient")
+                return grad_omega, grad_sigma, None, None, None
         grad_omega = (right_jacobian(w).transpose(-1, -2) @ grad_body[..., None])[..., 0]
         return grad_omega, grad_sigma, None, None, None
 

@@ -182,6 +182,17 @@ class Matcha:
         sigma, its Euler gradient (B, 3) and Hessian (B, 3, 3) (``mtb_score_derivatives``; the
         quantities of WignerDGradients.get_derivatives, WignerDGradients.py:247-302).
         L defaults to L_max; angles (B,) in radians."""
+        out = self.score_and_derivatives(sigma, alpha, beta, gamma, L)
+        h = out[:, 4:]
+        H = torch.stack([torch.stack([h[:, 0], h[:, 1], h[:, 2]], -1),
+                         torch.stack([h[:, 1], h[:, 3], h[:, 4]], -1),
+                         torch.stack([h[:, 2], h[:, 4], h[:, 5]], -1)], -2)
+        return out[:, 0], out[:, 1:4], H
+
+    @torch.no_grad()
+    def score_and_derivatives(self, sigma, alpha, beta, gamma, L: int = None):
+        """The rows ``mtb_score_derivatives`` writes, (B, 10): score, Euler gradient (a, b, g) and
+        Hessian (aa, ab, ag, bb, bg, gg)."""
         L = self.Lmax if L is None else int(L)
         if not 0 <= L <= self.Lmax:
             raise ValueError(f"L must be in [0, {self.Lmax}]")
@@ -205,11 +216,7 @@ class Matcha:
                                                       nat.ptr(ang[0]), nat.ptr(ang[1]), nat.ptr(ang[2]),
                                                       nat.ptr(out), nat.stream_ptr(sigma.device)),
                       "mtb_score_derivatives")
-        h = out[:, 4:]
-        H = torch.stack([torch.stack([h[:, 0], h[:, 1], h[:, 2]], -1),
-                         torch.stack([h[:, 1], h[:, 3], h[:, 4]], -1),
-                         torch.stack([h[:, 2], h[:, 4], h[:, 5]], -1)], -2)
-        return out[:, 0], out[:, 1:4], H
+        return out
 
     @torch.no_grad()
     def search_orientations(self, sigma):

@@ -333,6 +333,83 @@ sigma_backward_template_kernel(const float2* __restrict__ aV, int64_t v_stride, 
   }
 }
 
+// ------------------------------------------------------------------ rotations of a batch
+// exp([w]x) = I + a [w]x + b [w]x^2 and the right Jacobian I - c1 [w]x + c2 [w]x^2.
+__device__ __forceinline__ void so3_coefficients(double th2, double& a, double& b, double& c2) {
+  const double th = sqrt(th2);
+  if (th < 1e-6) {
+    a = 1.0 - th2 / 6.0;
+    b = 0.5 - th2 / 24.0;
+    c2 = 1.0 / 6.0 - th2 / 120.0;
+  } else {
+    double sn, cs;
+    sincos(th, &sn, &cs);
+    a = sn / th;
+    b = (1.0 - cs) / th2;
+    c2 = (th - sn) / (th2 * th);
+  }
+}
+
+// Euler angles of Rz(a) Ry(b) Rz(g) exp([omega]x), FP64 up to the FP32 angles.  One thread per
+// rotation: the batch's hundred small matrix operations in one launch.
+__global__ void rotation_angles_kernel(const double* __restrict__ omega, const double* __restrict__ base, int B,
+                                       float* __restrict__ alpha, float* __restrict__ beta, float* __restrict__ gamma) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= B) return;
+  const double x = omega[3 * i], y = omega[3 * i + 1], z = omega[3 * i + 2];
+  const double x2 = x * x, y2 = y * y, z2 = z * z;
+  double a, b, c2;
+  so3_coefficients(x2 + y2 + z2, a, b, c2);
+  const double E[3][3] = {{1.0 - b * (y2 + z2), b * x * y - a * z, b * x * z + a * y},
+                          {b * x * y + a * z, 1.0 - b * (x2 + z2), b * y * z - a * x},
+                          {b * x * z - a * y, b * y * z + a * x, 1.0 - b * (x2 + y2)}};
+  double sa, ca, sb, cb, sg, cg;
+  sincos(base[3 * i], &sa, &ca);
+  sincos(base[3 * i + 1], &sb, &cb);
+  sincos(base[3 * i + 2], &sg, &cg);
+  const double Z[3][3] = {{ca * cb * cg - sa * sg, -ca * cb * sg - sa * cg, ca * sb},
+                          {sa * cb * cg + ca * sg, -sa * cb * sg + ca * cg, sa * sb},
+                          {-sb * cg, sb * sg, cb}};
+  double R[3][3];
+#pragma unroll
+  for (int r = 0; r < 3; ++r)
+#pragma unroll
+    for (int c = 0; c < 3; ++c) R[r][c] = Z[r][0] * E[0][c] + Z[r][1] * E[1][c] + Z[r][2] * E[2][c];
+  const double s = sqrt(R[0][2] * R[0][2] + R[1][2] * R[1][2]);
+  double al, be, ga;
+  if (s < 1e-12) {  // beta = 0 or pi: only a + g or a - g is defined, g = 0
+    const bool up = R[2][2] > 0;
+    al = up ? atan2(R[1][0], R[0][0]) : atan2(-R[1][0], -R[0][0]);
+    be = up ? 0.0 : 3.14159265358979323846;
+    ga = 0.0;
+  } else {
+    al = atan2(R[1][2], R[0][2]);
+    be = atan2(s, R[2][2]);
+    ga = atan2(R[2][1], -R[2][0]);
+  }
+  alpha[i] = (float)al;
+  beta[i] = (float)be;
+  gamma[i] = (float)ga;
+}
+
+// grad_omega = Jr(omega)^T grad_body.
+__global__ void rotation_gradient_kernel(const double* __restrict__ omega, const double* __restrict__ grad_body, int B,
+                                         double* __restrict__ grad_omega) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= B) return;
+  const double x = omega[3 * i], y = omega[3 * i + 1], z = omega[3 * i + 2];
+  const double x2 = x * x, y2 = y * y, z2 = z * z;
+  double a, c1, c2;
+  so3_coefficients(x2 + y2 + z2, a, c1, c2);
+  // rows of Jr = I - c1 [w]x + c2 [w]x^2, transposed on the way out
+  const double J[3][3] = {{1.0 - c2 * (y2 + z2), c2 * x * y + c1 * z, c2 * x * z - c1 * y},
+                          {c2 * x * y - c1 * z, 1.0 - c2 * (x2 + z2), c2 * y * z + c1 * x},
+                          {c2 * x * z + c1 * y, c2 * y * z - c1 * x, 1.0 - c2 * (x2 + y2)}};
+  const double g[3] = {grad_body[3 * i], grad_body[3 * i + 1], grad_body[3 * i + 2]};
+#pragma unroll
+  for (int c = 0; c < 3; ++c) grad_omega[3 * i + c] = J[0][c] * g[0] + J[1][c] * g[1] + J[2][c] * g[2];
+}
+
 }  // namespace
 
 extern "C" int mtb_score_backward(const float* sigma, int64_t sigma_stride, int B, int L, const float* alpha,
@@ -407,6 +484,32 @@ extern "C" int mtb_sigma_backward_template(mtb_fle* h, const float* coeffs, int6
       reinterpret_cast<const float2*>(coeffs), coeff_stride, reinterpret_cast<const float2*>(grad_sigma), grad_stride,
       B, lmax_g, n_sub, (int)(rows / sizeof(float2)), kpad, koff, kidx, reinterpret_cast<float2*>(grad_tmpl));
   mtb_prof_end(st, "sigma_backward_template_kernel");
+  MTB_LAUNCH_CHECK();
+  return MTB_OK;
+}
+
+extern "C" int mtb_rotation_angles(const double* omega, const double* base, int B, float* alpha, float* beta,
+                                   float* gamma, mtb_stream_t stream) {
+  MTB_ARG_CHECK(B >= 0, "negative batch");
+  if (B == 0) return MTB_OK;
+  MTB_ARG_CHECK(omega && base && alpha && beta && gamma, "null pointer");
+  const cudaStream_t st = (cudaStream_t)stream;
+  mtb_prof_begin(st);
+  rotation_angles_kernel<<<(B + 63) / 64, 64, 0, st>>>(omega, base, B, alpha, beta, gamma);
+  mtb_prof_end(st, "rotation_angles_kernel");
+  MTB_LAUNCH_CHECK();
+  return MTB_OK;
+}
+
+extern "C" int mtb_rotation_gradient(const double* omega, const double* grad_body, int B, double* grad_omega,
+                                     mtb_stream_t stream) {
+  MTB_ARG_CHECK(B >= 0, "negative batch");
+  if (B == 0) return MTB_OK;
+  MTB_ARG_CHECK(omega && grad_body && grad_omega, "null pointer");
+  const cudaStream_t st = (cudaStream_t)stream;
+  mtb_prof_begin(st);
+  rotation_gradient_kernel<<<(B + 63) / 64, 64, 0, st>>>(omega, grad_body, B, grad_omega);
+  mtb_prof_end(st, "rotation_gradient_kernel");
   MTB_LAUNCH_CHECK();
   return MTB_OK;
 }

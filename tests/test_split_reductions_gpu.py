@@ -97,3 +97,32 @@ def test_shift_score_gradient(cuda_device, N, B):
         # the FP32 transforms in front of the sum: 2e-5 of the score's scale (unit-norm products)
         assert abs(c[b].item() - c_ref) < 2e-5
         np.testing.assert_allclose(g[b].cpu().numpy(), g_ref, rtol=0, atol=2e-5 * np.pi)
+
+
+@pytest.mark.parametrize("B", [1, 63, 64, 65, 200])
+def test_rotation_angles_and_gradient(cuda_device, B):
+    """The one-launch rotations against the module's own torch functions in FP64: the rotation of
+    the angles within FP32 rounding of angles up to pi (2e-7 each), the gradient in FP64."""
+    from matcha_b200 import _native as nat
+    from matcha_b200.autograd import right_jacobian, so3_exp, zyz_matrix
+
+    rng = np.random.default_rng(B)
+    omega, base = torch.tensor(rng.standard_normal((B, 3))), torch.tensor(rng.uniform(-3, 3, (B, 3)))
+    omega[0] = 0
+    base[0, 1] = 0.0
+    if B > 2:
+        omega[1], base[1, 1] = 0, np.pi
+        omega[2] = torch.tensor([1e-9, -2e-9, 1e-7], dtype=torch.float64)
+    body = torch.tensor(rng.standard_normal((B, 3)))
+    w, e, g = (t.to(cuda_device) for t in (omega, base, body))
+    ang, out = torch.empty((3, B), device=cuda_device), torch.empty_like(w)
+    lib = nat.load()
+    nat.check(lib.mtb_rotation_angles(nat.ptr(w), nat.ptr(e), B, nat.ptr(ang[0]), nat.ptr(ang[1]), nat.ptr(ang[2]),
+                                      nat.stream_ptr(cuda_device)), "mtb_rotation_angles")
+    nat.check(lib.mtb_rotation_gradient(nat.ptr(w), nat.ptr(g), B, nat.ptr(out), nat.stream_ptr(cuda_device)),
+              "mtb_rotation_gradient")
+    R = zyz_matrix(base[:, 0], base[:, 1], base[:, 2]) @ so3_exp(omega)
+    torch.testing.assert_close(zyz_matrix(*ang.cpu().double()), R, atol=1e-6, rtol=0)
+    assert bool((ang[1] >= 0).all())
+    ref = (right_jacobian(omega).transpose(-1, -2) @ body[..., None])[..., 0]
+    torch.testing.assert_close(out.cpu(), ref, atol=1e-9, rtol=0)
