@@ -39,13 +39,21 @@ constexpr int kNT = kNewtonThreads;
 
 enum { A_VAL = 0, A_GA, A_GB, A_GG, A_HAA, A_HAB, A_HAG, A_HBB, A_HBG, A_HGG, A_N };
 
+// A candidate's point with what a pass needs of it.
+struct Point {
+  double hs, hc;       // sin, cos of beta / 2
+  float a, be, ga;
+  float sb, cb;        // sin, cos of beta
+};
+
 // Per-candidate tables of one pass (NC candidates of one subtomogram per CTA).
 template <int NC>
 struct Smem {
-  float2 (*ea)[2 * kNewtonMaxL + 1];   // e^{i k a}, index k + Li
-  float2 (*eg)[2 * kNewtonMaxL + 1];   // e^{i k g}, index k + Li
+  float2 (*ea)[kNewtonMaxL + 1];       // e^{i k a}, k = 0 .. Li
+  float2 (*eg)[kNewtonMaxL + 1];       // e^{i k g}
   double (*phc)[2 * kNewtonMaxL + 3];  // cos(b/2)^k, k = 0 .. 2 Li + 2
   double (*pt)[2 * kNewtonMaxL + 3];   // (-sin(b/2))^k
+  uint32_t* off;                       // 16 wedge_off(l): byte offset of degree l
   float* red;                          // (threads/32) x NC x A_N
   float* res;                          // NC x A_N
 };
@@ -128,51 +136,100 @@ __global__ void coef_kernel(int64_t n, float4* __restrict__ coef) {
   }
 }
 
-__device__ __forceinline__ float2 cmulf(float2 a, float2 b) {
-  return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+// The point of a candidate: its trigonometric values, once for the CTA.
+__device__ __forceinline__ Point make_point(float a, float be, float ga) {
+  Point p;
+  p.a = a;
+  p.be = be;
+  p.ga = ga;
+  sincos(0.5 * (double)be, &p.hs, &p.hc);
+  sincosf(be, &p.sb, &p.cb);
+  return p;
 }
 
-// One sweep over the chains of stage degree Li at the NC points (a[c], be[c], ga[c]) of one
-// subtomogram's candidates: value, and with DERIVS the Euler gradient and Hessian, left in
+__device__ __forceinline__ const float4* at_bytes(const float4* base, uint32_t off) {
+  return reinterpret_cast<const float4*>(reinterpret_cast<const char*>(base) + off);
+}
+
+// Sums of N values over a warp, each by the tree of an exchange between lanes 16, 8, 4, 2 and 1
+// apart.  While a lane holds an even number of values it hands half of them over and keeps the
+// other half's sums, so the 20 values of a pass cost 30 exchanges instead of 100; a value's
+// additions are the same.  out[i] receives the sum of value i.
+template <int N, int O>
+struct WarpSums {
+  static __device__ __forceinline__ void run(float (&x)[N], int lane, int first, float* out) {
+    if constexpr (O >= 1 && N % 2 == 0) {
+      constexpr int M = N / 2;
+      const bool up = lane & O;
+      float y[M];
+#pragma unroll
+      for (int j = 0; j < M; ++j) {
+        const float give = up ? x[j] : x[j + M], keep = up ? x[j + M] : x[j];
+        y[j] = keep + __shfl_xor_sync(0xffffffffu, give, O);
+      }
+      first += up ? M : 0;
+      WarpSums<M, O / 2>::run(y, lane, first, out);
+    } else {
+#pragma unroll
+      for (int o = O; o > 0; o >>= 1)
+#pragma unroll
+        for (int j = 0; j < N; ++j) x[j] += __shfl_xor_sync(0xffffffffu, x[j], o);
+      if ((lane & (2 * O - 1)) == 0)
+#pragma unroll
+        for (int j = 0; j < N; ++j) out[first + j] = x[j];
+    }
+  }
+};
+
+__device__ __forceinline__ float2 cmulf(float2 a, float2 b) {
+  return make_float2(__fmaf_rn(a.x, b.x, -__fmul_rn(a.y, b.y)), __fmaf_rn(a.y, b.x, __fmul_rn(a.x, b.y)));
+}
+
+// One sweep over the chains of stage degree Li at the NC points pts[c] of one subtomogram's
+// candidates: value, and with DERIVS the Euler gradient and Hessian, left in
 // sm.res[c * A_N + ..].  The candidates share each chain's loads of the folded sigma and of
 // the recurrence factors; their d, d', d'' run side by side.  FOLDED reads the folded sigma S
 // of this subtomogram; otherwise each step folds the four images from sigma itself.
+//
+// Issue bounds it, and of the 24 M thread instructions a subtomogram took at L = 32 only a third
+// were FP32; so everything around the chain steps is kept short: the points' trigonometry and the
+// FP64 step are one thread's, tables hold k >= 0 and are filled by all threads, offsets are 32-bit,
+// the sums of a warp are exchanged by halves.  March of 1000 subtomograms at L = 32 1104 -> 884 us,
+// 64 at L = 64 608 -> 509 us, 16 at L = 16 (five steps) 86 -> 50 us.  (A cp.async ring of four steps
+// per thread instead of plain loads measured 1196 and 543 us before these; 96 registers and five
+// CTAs per SM 890 and 704 us.)
 template <bool DERIVS, bool FOLDED, int NC>
 __device__ __forceinline__ void pass(const float4* __restrict__ S, const float2* __restrict__ sg,
                                      const float4* __restrict__ coef, const double* __restrict__ Ctab,
-                                     const float (&a)[NC], const float (&be)[NC], const float (&ga)[NC], int Li,
-                                     const Smem<NC> sm) {
+                                     const Point* pts, int Li, const Smem<NC> sm) {
   const int tid = threadIdx.x;
   const double two_pi = 6.283185307179586;
-#pragma unroll
-  for (int c = 0; c < NC; ++c) {
-    for (int r = tid; r < 2 * Li + 1; r += kNT) {
-      double t = (double)(r - Li) * (double)a[c];
-      t -= two_pi * rint(t / two_pi);
-      float s, co;
-      sincosf((float)t, &s, &co);
-      sm.ea[c][r] = make_float2(co, s);
-      t = (double)(r - Li) * (double)ga[c];
-      t -= two_pi * rint(t / two_pi);
-      sincosf((float)t, &s, &co);
-      sm.eg[c][r] = make_float2(co, s);
-    }
-    double hs, hc;
-    sincos(0.5 * (double)be[c], &hs, &hc);
-    for (int k = tid; k <= 2 * Li + 2; k += kNT) {
-      sm.phc[c][k] = ipow(hc, k);
-      sm.pt[c][k] = ipow(-hs, k);
-    }
+  for (int e = tid; e < NC * 2 * (Li + 1); e += kNT) {
+    const int c = e / (2 * (Li + 1)), r = e - c * (2 * (Li + 1)), g = r > Li, k = r - g * (Li + 1);
+    double t = (double)k * (double)(g ? pts[c].ga : pts[c].a);
+    t -= two_pi * rint(t / two_pi);
+    float s, co;
+    sincosf((float)t, &s, &co);
+    (g ? sm.eg : sm.ea)[c][k] = make_float2(co, s);
+  }
+  const int np = DERIVS ? 2 * Li + 3 : 2 * Li + 1;
+  for (int e = tid; e < NC * 2 * np; e += kNT) {
+    const int c = e / (2 * np), r = e - c * (2 * np), h = r >= np, k = r - h * np;
+    (h ? sm.pt : sm.phc)[c][k] = ipow(h ? -pts[c].hs : pts[c].hc, k);
   }
   float sb[NC], cb[NC];
 #pragma unroll
-  for (int c = 0; c < NC; ++c) sincosf(be[c], &sb[c], &cb[c]);
+  for (int c = 0; c < NC; ++c) {
+    sb[c] = pts[c].sb;
+    cb[c] = pts[c].cb;
+  }
 
-  float acc[NC][A_N];
+  constexpr int NA = DERIVS ? A_N : 1;
+  float acc[NC][NA];
 #pragma unroll
   for (int c = 0; c < NC; ++c)
 #pragma unroll
-    for (int i = 0; i < A_N; ++i) acc[c][i] = 0.f;
+    for (int i = 0; i < NA; ++i) acc[c][i] = 0.f;
   __syncthreads();
 
   const int n = (Li + 1) * (Li + 1);
@@ -180,8 +237,9 @@ __device__ __forceinline__ void pass(const float4* __restrict__ S, const float2*
   for (int base = 0; base < n; base += kNT, ++k) {
     const int p = base + ((k & 1) ? kNT - 1 - tid : tid);
     if (p >= n) continue;
-    int mp, m;
-    wedge_pair(p, mp, m);
+    float root;
+    asm("sqrt.approx.f32 %0, %1;" : "=f"(root) : "f"((float)p + 0.5f));
+    const int mp = (int)root, m = p - mp * mp - mp;  // wedge_pair (the half keeps the root off integers)
     // start of the chain at l = M': d = C cos^P (-sin)^Q of b/2, P = M'+M, Q = M'-M
     const int P = mp + m, Q = mp - m;
     const double Cp = Ctab[p];
@@ -201,8 +259,9 @@ __device__ __forceinline__ void pass(const float4* __restrict__ S, const float2*
         g1[c] = (float)(0.25 * Cp * fpp);
       }
     }
+    uint32_t off = sm.off[mp] + 16u * (uint32_t)p;
     float4 s;
-    if (FOLDED) s = __ldg(S + wedge_off(mp) + p);
+    if (FOLDED) s = __ldg(at_bytes(S, off));
     else s = fold_entry(sg, mp, mp, m);
     // per candidate: A = sum d S (a1 = S1 part, a2 = S2 part), B = sum d' S, C = sum d'' S
     float A1r[NC], A1i[NC], A2r[NC], A2i[NC];
@@ -216,13 +275,8 @@ __device__ __forceinline__ void pass(const float4* __restrict__ S, const float2*
         C1r[c] = g1[c] * s.x; C1i[c] = g1[c] * s.y; C2r[c] = g1[c] * s.z; C2i[c] = g1[c] * s.w;
       }
     }
-    const float4* cp = coef + wedge_off(mp + 1) + p;
-    const float4* sp = FOLDED ? S + wedge_off(mp + 1) + p : nullptr;
-#pragma unroll 4
-    for (int l = mp + 1; l <= Li; ++l) {
-      const float4 cf = __ldg(cp);
-      if (FOLDED) s = __ldg(sp);
-      else s = fold_entry(sg, l, mp, m);
+    // one chain step from its recurrence factors and folded sigma
+    auto step = [&](const float4 cf, const float4 s) {
 #pragma unroll
       for (int c = 0; c < NC; ++c) {
         const float t = fmaf(cf.x, cb[c], -cf.y);
@@ -244,30 +298,49 @@ __device__ __forceinline__ void pass(const float4* __restrict__ S, const float2*
           C2r[c] = fmaf(g1[c], s.z, C2r[c]); C2i[c] = fmaf(g1[c], s.w, C2i[c]);
         }
       }
-      cp += (l + 1) * (l + 1);
-      if (FOLDED) sp += (l + 1) * (l + 1);
+    };
+    // degree l + 1 lies 16 (l + 1)^2 bytes after degree l
+    uint32_t inc = 16u * (uint32_t)((mp + 1) * (mp + 1)), grow = 16u * (uint32_t)(2 * mp + 3);
+    off += inc;
+#pragma unroll 4
+    for (int l = mp + 1; l <= Li; ++l) {
+      const float4 cf = __ldg(at_bytes(coef, off));
+      step(cf, FOLDED ? __ldg(at_bytes(S, off)) : fold_entry(sg, l, mp, m));
+      inc += grow;
+      grow += 32u;
+      off += inc;
     }
     // phases: z1 = e^{i(M'a + Mg)}, z2 = e^{i(Ma + M'g)}
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
-      const float2 z1 = cmulf(sm.ea[c][mp + Li], sm.eg[c][m + Li]);
-      const float2 z2 = cmulf(sm.ea[c][m + Li], sm.eg[c][mp + Li]);
+      const int am = abs(m);
+      float2 eam = sm.ea[c][am], egm = sm.eg[c][am];
+      if (m < 0) {
+        eam.y = -eam.y;
+        egm.y = -egm.y;
+      }
+      const float2 z1 = cmulf(sm.ea[c][mp], egm);
+      const float2 z2 = cmulf(eam, sm.eg[c][mp]);
       const float r1 = z1.x * A1r[c] - z1.y * A1i[c], r2 = z2.x * A2r[c] - z2.y * A2i[c];
       acc[c][A_VAL] += r1 + r2;
       if (DERIVS) {
         const float fM = (float)mp, fm = (float)m;
-        const float j1 = z1.x * A1i[c] + z1.y * A1r[c], j2 = z2.x * A2i[c] + z2.y * A2r[c];
+        // which product of a pair is fused is written out, so that the one- and two-candidate
+        // kernels, and later compilers, round alike
+        auto imag = [](float2 z, float r, float i) { return __fmaf_rn(z.x, i, __fmul_rn(z.y, r)); };
+        auto lin = [](float x, float u, float y, float v) { return __fmaf_rn(x, u, __fmul_rn(y, v)); };
+        const float j1 = imag(z1, A1r[c], A1i[c]), j2 = imag(z2, A2r[c], A2i[c]);
         const float q1 = z1.x * B1r[c] - z1.y * B1i[c], q2 = z2.x * B2r[c] - z2.y * B2i[c];
-        const float k1 = z1.x * B1i[c] + z1.y * B1r[c], k2 = z2.x * B2i[c] + z2.y * B2r[c];
+        const float k1 = imag(z1, B1r[c], B1i[c]), k2 = imag(z2, B2r[c], B2i[c]);
         const float h1 = z1.x * C1r[c] - z1.y * C1i[c], h2 = z2.x * C2r[c] - z2.y * C2i[c];
-        acc[c][A_GA] -= fM * j1 + fm * j2;
-        acc[c][A_GG] -= fm * j1 + fM * j2;
+        acc[c][A_GA] -= lin(fM, j1, fm, j2);
+        acc[c][A_GG] -= lin(fm, j1, fM, j2);
         acc[c][A_GB] += q1 + q2;
         acc[c][A_HAA] -= fM * fM * r1 + fm * fm * r2;
         acc[c][A_HGG] -= fm * fm * r1 + fM * fM * r2;
         acc[c][A_HAG] -= fM * fm * (r1 + r2);
-        acc[c][A_HAB] -= fM * k1 + fm * k2;
-        acc[c][A_HBG] -= fm * k1 + fM * k2;
+        acc[c][A_HAB] -= lin(fM, k1, fm, k2);
+        acc[c][A_HBG] -= lin(fm, k1, fM, k2);
         acc[c][A_HBB] += h1 + h2;
       }
     }
@@ -275,20 +348,20 @@ __device__ __forceinline__ void pass(const float4* __restrict__ S, const float2*
 
   // ---- block reduction
   const int lane = tid & 31, warp = tid >> 5;
-  constexpr int NA = DERIVS ? A_N : 1;
+  {
+    float x[NC * NA];
 #pragma unroll
-  for (int c = 0; c < NC; ++c)
+    for (int c = 0; c < NC; ++c)
 #pragma unroll
-    for (int i = 0; i < NA; ++i) {
-      const float v = warp_sum(acc[c][i]);
-      if (lane == 0) sm.red[(warp * NC + c) * A_N + i] = v;
-    }
+      for (int i = 0; i < NA; ++i) x[c * NA + i] = acc[c][i];
+    WarpSums<NC * NA, 16>::run(x, lane, 0, sm.red + warp * NC * A_N);
+  }
   __syncthreads();
   if (tid < NC * A_N) {
     const int c = tid / A_N, i = tid - (tid / A_N) * A_N;
     if (i < NA) {
       float s2 = 0.f;
-      for (int q = 0; q < kNT / 32; ++q) s2 += sm.red[(q * NC + c) * A_N + i];
+      for (int q = 0; q < kNT / 32; ++q) s2 += sm.red[q * NC * A_N + c * NA + i];
       sm.res[c * A_N + i] = s2;
     }
   }
@@ -332,10 +405,12 @@ newton_march_kernel(const float4* __restrict__ S, int64_t n_fold, const float2* 
                     int BC, int C, float* __restrict__ alpha, float* __restrict__ beta, float* __restrict__ gamma,
                     float* __restrict__ score, const double* __restrict__ Ctab, const float4* __restrict__ coef,
                     NewtonParams P) {
-  __shared__ float2 s_ea[NC][2 * kNewtonMaxL + 1], s_eg[NC][2 * kNewtonMaxL + 1];
+  __shared__ float2 s_ea[NC][kNewtonMaxL + 1], s_eg[NC][kNewtonMaxL + 1];
   __shared__ double s_phc[NC][2 * kNewtonMaxL + 3], s_pt[NC][2 * kNewtonMaxL + 3];
+  __shared__ uint32_t s_off[kNewtonMaxL + 1];
   __shared__ float s_red[(kNT / 32) * NC * A_N], s_res[NC * A_N];
-  const Smem<NC> sm{s_ea, s_eg, s_phc, s_pt, s_red, s_res};
+  __shared__ Point s_now[NC], s_try[NC];  // each candidate's accepted and trial point
+  const Smem<NC> sm{s_ea, s_eg, s_phc, s_pt, s_off, s_red, s_res};
 
   const int cand0 = blockIdx.x * NC;
   if (cand0 >= BC) return;
@@ -344,92 +419,77 @@ newton_march_kernel(const float4* __restrict__ S, int64_t n_fold, const float2* 
   const float2* sg = FOLDED ? nullptr : sigma + (int64_t)b * stride;
   const bool grad_step = (P.flags & MTB_SEARCH_GRADIENT_STEP) != 0;
   const float base_lr = grad_step ? 5e-7f : 1.f;
+  for (int l = threadIdx.x; l <= P.Lmax; l += kNT) s_off[l] = 16u * (uint32_t)wedge_off(l);
 
-  // the gradient and Hessian at each candidate's accepted point: pass results (res layout),
-  // kept in shared memory so they are not live in registers across the passes
-  __shared__ float s_gh[NC * A_N];
-  float a[NC], be[NC], ga[NC], best[NC];
-#pragma unroll
-  for (int c = 0; c < NC; ++c) {
-    a[c] = alpha[cand0 + c];
-    be[c] = beta[cand0 + c];
-    ga[c] = gamma[cand0 + c];
-    best[c] = 0.f;
-  }
+  // candidate c's state (best score, learning rate, gradient and Hessian at the accepted point)
+  // is one thread's, in a warp of its own: it takes the FP64 step while the other CTAs of the SM
+  // have the issue slots
+  const int c = threadIdx.x >> 5;
+  const bool owner = (threadIdx.x & 31) == 0 && c < NC;
+  // (in shared memory: registers would be live across the passes)
+  __shared__ float s_gh[NC][A_N], s_best[NC], s_lr[NC];
+  float* gh = s_gh[owner ? c : 0];
+  if (owner) s_now[c] = make_point(alpha[cand0 + c], beta[cand0 + c], gamma[cand0 + c]);
+  __syncthreads();
   for (int st = 0; st < P.n_stages; ++st) {
     const int Li = P.stages[st];
     if (P.num_steps > 0)
-      pass<true, FOLDED, NC>(Sb, sg, coef, Ctab, a, be, ga, Li, sm);
+      pass<true, FOLDED, NC>(Sb, sg, coef, Ctab, s_now, Li, sm);
     else
-      pass<false, FOLDED, NC>(Sb, sg, coef, Ctab, a, be, ga, Li, sm);
-    float lr[NC];
+      pass<false, FOLDED, NC>(Sb, sg, coef, Ctab, s_now, Li, sm);
+    if (owner) {
 #pragma unroll
-    for (int c = 0; c < NC; ++c) {
-      best[c] = sm.res[c * A_N + A_VAL];
-      lr[c] = base_lr;
+      for (int i = 0; i < A_N; ++i) gh[i] = s_res[c * A_N + i];
+      s_best[c] = gh[A_VAL];
+      s_lr[c] = base_lr;
     }
-    if (threadIdx.x < NC * A_N) s_gh[threadIdx.x] = sm.res[threadIdx.x];
-    __syncthreads();
     for (int it = 0; it < P.num_steps; ++it) {
-      float ta[NC], tb[NC], tg[NC];
-#pragma unroll
-      for (int c = 0; c < NC; ++c) {
-        const float* r = s_gh + c * A_N;
-        const double g[3] = {r[A_GA], r[A_GB], r[A_GG]};
-        const double H[3][3] = {{r[A_HAA], r[A_HAB], r[A_HAG]},
-                                {r[A_HAB], r[A_HBB], r[A_HBG]},
-                                {r[A_HAG], r[A_HBG], r[A_HGG]}};
+      if (owner) {
+        const double g[3] = {gh[A_GA], gh[A_GB], gh[A_GG]};
+        const double H[3][3] = {{gh[A_HAA], gh[A_HAB], gh[A_HAG]},
+                                {gh[A_HAB], gh[A_HBB], gh[A_HBG]},
+                                {gh[A_HAG], gh[A_HBG], gh[A_HGG]}};
         double x[3] = {0.0, 0.0, 0.0};
         if (grad_step) {
           for (int i = 0; i < 3; ++i) x[i] = -g[i];
         } else if (!solve3(H, g, x)) {
           x[0] = x[1] = x[2] = 0.0;
         }
-        ta[c] = a[c] - lr[c] * (float)x[0];
-        tb[c] = be[c] - lr[c] * (float)x[1];
-        tg[c] = ga[c] - lr[c] * (float)x[2];
+        const Point now = s_now[c];
+        const float lr = s_lr[c];
+        const float ta = now.a - lr * (float)x[0];
+        const float tb = now.be - lr * (float)x[1];
+        const float tg = now.ga - lr * (float)x[2];
+        s_try[c] = make_point(ta, tb, tg);
       }
+      __syncthreads();
       const bool last = (it == P.num_steps - 1);
-      __syncthreads();  // everyone has read the previous results
       if (last)
-        pass<false, FOLDED, NC>(Sb, sg, coef, Ctab, ta, tb, tg, Li, sm);
+        pass<false, FOLDED, NC>(Sb, sg, coef, Ctab, s_try, Li, sm);
       else
-        pass<true, FOLDED, NC>(Sb, sg, coef, Ctab, ta, tb, tg, Li, sm);
-      bool took[NC];
+        pass<true, FOLDED, NC>(Sb, sg, coef, Ctab, s_try, Li, sm);
+      if (owner) {
+        const float ev = s_res[c * A_N + A_VAL];
+        if (ev > s_best[c]) {
+          s_now[c] = s_try[c];
+          s_best[c] = ev;
+          s_lr[c] *= 1.1f;
+          if (!last) {
 #pragma unroll
-      for (int c = 0; c < NC; ++c) {
-        const float ev = sm.res[c * A_N + A_VAL];
-        took[c] = ev > best[c];
-        if (took[c]) {
-          a[c] = ta[c]; be[c] = tb[c]; ga[c] = tg[c]; best[c] = ev;
-          lr[c] *= 1.1f;
+            for (int i = 0; i < A_N; ++i) gh[i] = s_res[c * A_N + i];
+          }
         } else {
-          lr[c] *= 0.5f;
+          s_lr[c] *= 0.5f;
         }
-      }
-      if (!last) {
-        if (threadIdx.x < NC * A_N) {
-          const int c = threadIdx.x / A_N;
-          bool tk = false;
-#pragma unroll
-          for (int q = 0; q < NC; ++q) tk = (q == c) ? took[q] : tk;
-          if (tk) s_gh[threadIdx.x] = sm.res[threadIdx.x];
-        }
-        __syncthreads();
       }
     }
-    __syncthreads();
+    __syncthreads();  // the accepted points, before the next stage's pass
   }
-  if (threadIdx.x < NC) {
-    const int c = threadIdx.x;
-#pragma unroll
-    for (int q = 0; q < NC; ++q)
-      if (q == c) {
-        alpha[cand0 + c] = a[q];
-        beta[cand0 + c] = be[q];
-        gamma[cand0 + c] = ga[q];
-        score[cand0 + c] = best[q];
-      }
+  if (owner) {
+    alpha[cand0 + c] = s_now[c].a;
+    beta[cand0 + c] = s_now[c].be;
+    gamma[cand0 + c] = s_now[c].ga;
+    score[cand0 + c] = s_best[c];
   }
 }
 
@@ -440,13 +500,17 @@ __global__ void __launch_bounds__(kNT)
 score_derivs_kernel(const float2* __restrict__ sigma, int64_t stride, const float* __restrict__ alpha,
                     const float* __restrict__ beta, const float* __restrict__ gamma, int Li,
                     const double* __restrict__ Ctab, const float4* __restrict__ coef, float* __restrict__ out) {
-  __shared__ float2 s_ea[1][2 * kNewtonMaxL + 1], s_eg[1][2 * kNewtonMaxL + 1];
+  __shared__ float2 s_ea[1][kNewtonMaxL + 1], s_eg[1][kNewtonMaxL + 1];
   __shared__ double s_phc[1][2 * kNewtonMaxL + 3], s_pt[1][2 * kNewtonMaxL + 3];
+  __shared__ uint32_t s_off[kNewtonMaxL + 1];
   __shared__ float s_red[(kNT / 32) * A_N], s_res[A_N];
-  const Smem<1> sm{s_ea, s_eg, s_phc, s_pt, s_red, s_res};
+  __shared__ Point s_now[1];
+  const Smem<1> sm{s_ea, s_eg, s_phc, s_pt, s_off, s_red, s_res};
   const int b = blockIdx.x;
-  const float a[1] = {alpha[b]}, be[1] = {beta[b]}, ga[1] = {gamma[b]};
-  pass<true, false, 1>(nullptr, sigma + (int64_t)b * stride, coef, Ctab, a, be, ga, Li, sm);
+  for (int l = threadIdx.x; l <= Li; l += kNT) s_off[l] = 16u * (uint32_t)wedge_off(l);
+  if (threadIdx.x == 0) s_now[0] = make_point(alpha[b], beta[b], gamma[b]);
+  __syncthreads();
+  pass<true, false, 1>(nullptr, sigma + (int64_t)b * stride, coef, Ctab, s_now, Li, sm);
   if (threadIdx.x < A_N) out[(int64_t)b * A_N + threadIdx.x] = sm.res[threadIdx.x];
 }
 
@@ -482,8 +546,10 @@ int newton_launch(const float* sigma, int64_t stride, int B, int C, float* a, fl
   const int BC = B * C;
   const float2* sg = reinterpret_cast<const float2*>(sigma);
   const int64_t nf = newton_fold_entries(P.Lmax);
-  // two candidates of a subtomogram per CTA share its folded-sigma and recurrence-factor loads
-  const bool pair = (C % 2) == 0;
+  // two candidates of a subtomogram per CTA share its folded-sigma and recurrence-factor loads,
+  // where that still leaves a CTA per SM (16 subtomograms at L = 16: one each 50 us, two 56; 64 at
+  // L = 64: one 713, two 509)
+  const bool pair = (C % 2) == 0 && BC / 2 >= 148;
   if (fold) {
     mtb_prof_begin(st);
     fold_sigma_kernel<<<dim3(P.Lmax + 1, B), 256, 0, st>>>(sg, stride, nf, fold);
