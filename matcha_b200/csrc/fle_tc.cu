@@ -14,8 +14,8 @@
 // The second is for a basis that does not stay in L2 (64^3 up: 500 MB), where the loads, into
 // shared memory and from DRAM, set the pace; below, where the whole GEMM takes tens of us, the
 // first.  Times of the GEMM, before (segmented, one CTA per tile) and now: 1000 subtomograms of
-// 64^3 679 -> 545 us (1.47 PFLOP/s issued), 100 of 96^3 1397 -> 1187 us (5.1 TB/s of basis), 256 of
-// 64^3 324 -> 223 us, one of 48^3 85 -> 37 us.
+// 64^3 679 -> 550 us (1.46 PFLOP/s issued), 100 of 96^3 1397 -> 1105 us (5.5 TB/s of basis), 256 of
+// 64^3 321 -> 177 us, one of 64^3 291 -> 102 us, 128 of 48^3 138 -> 66 us, one of 48^3 118 -> 38 us.
 //
 // Accumulation: the tensor core adds each K=16 product into the FP32 accumulator with a
 // truncating alignment, an error of about one unit in the last place of the accumulator per
@@ -38,9 +38,9 @@
 // subtomograms of 96^3).
 //
 // Work units: the tiles that fill whole rounds of the 148 SMs are one CTA each; the rest are cut
-// along K into parts of q chunks (gemm_plan).  The first part of a tile leaves its sums in C, the
-// others leave theirs in slabs (one per chunk, or one per part in the interleaved order), and the
-// part that arrives last adds the slabs to C in order.  With a slab per chunk the additions are
+// along K into parts of q chunks (gemm_plan).  The first part of a tile leaves its sums in a slab,
+// the others theirs in more (one per chunk, or one per part in the interleaved order), and the
+// part that arrives last adds them in order.  With a slab per chunk the additions are
 // those of a whole tile, so a coefficient does not depend on the split, nor on the batch it is in.
 //
 // Every mbarrier wait is bounded; on expiry the kernel records an error code, stops
@@ -263,8 +263,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
     const int row = q * 32 + lane;
     const bool valid = m0 + row < P.M;
     const int ncol = min(tn, P.ncols[cls] - n0);  // valid columns of the tile
-    // slab column 0 of this thread's row and half; chunk c of a part after the first goes to slot
-    // c - q, or the whole part to slot part - 1
+    // slab column 0 of this thread's row and half; slot 0 takes the first part, 1 + c - q chunk c
+    // of a later one, or slot part the whole later part
     float* slab = P.slab + ((int64_t)(tile - P.whole) * P.slots * TN + h * (TN / 2)) * TM + row;
     float acc[TN / 2];
 #pragma unroll
@@ -281,7 +281,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * TN + h * (TN / 2));
       const bool to_slab = !INTERLEAVED && part > 0;
-      float* out = slab + (int64_t)(c - P.q) * TN * TM;
+      float* out = slab + (int64_t)(1 + c - P.q) * TN * TM;
 #pragma unroll
       for (int cb = 0; cb < TN / 2; cb += 32) {
         uint32_t v[32];
@@ -310,53 +310,74 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
       mbar_arrive_cta(&acc_empty[buf]);
     }
     float* crow = C + (int64_t)(m0 + row) * P.ldc + P.coff[cls] + n0 + h * (TN / 2);
-    if (done && valid) {
-      if (part == 0) {
+    const int w = min(TN / 2, ncol - h * (TN / 2));  // valid columns of this half (may be < 0)
+    if (done && valid && (part == 0 || INTERLEAVED)) {
+      const bool direct = !is_split || P.parts == 1;
+      float* out = direct ? crow : slab + (int64_t)part * TN * TM;
+      const int step = direct ? 1 : TM;
 #pragma unroll
-        for (int t = 0; t < TN / 2; ++t)
-          if (h * (TN / 2) + t < ncol) crow[t] = acc[t];
-      } else if (INTERLEAVED) {
-        float* out = slab + (int64_t)(part - 1) * TN * TM;
-#pragma unroll
-        for (int t = 0; t < TN / 2; ++t)
-          if (h * (TN / 2) + t < ncol) out[t * TM] = acc[t];
-      }
+      for (int t = 0; t < TN / 2; ++t)
+        if (t < w) out[t * step] = acc[t];
     }
     if (is_split && P.parts > 1) {
-      // the part that arrives last adds the slabs to C, in order (a part that gave up does not
-      // arrive: the call has failed then)
+      // the part that arrives last adds the slots in order (a part that gave up does not arrive: the
+      // call has failed then)
       __threadfence();
       asm volatile("bar.sync 1, %0;" ::"n"(kEpiThreads) : "memory");
-      if (threadIdx.x == 64) {
-        const int total = (nchunks + P.q - 1) / P.q;
-        last_part = !abort_flag && atomicAdd(&P.count[tile - P.whole], 1) == total - 1;
-      }
+      const int arrivals = (nchunks + P.q - 1) / P.q;
+      if (threadIdx.x == 64)
+        last_part = !abort_flag && atomicAdd(&P.count[tile - P.whole], 1) == arrivals - 1;
       asm volatile("bar.sync 1, %0;" ::"n"(kEpiThreads) : "memory");
-      if (last_part) {
-        __threadfence();
-        const int slots = INTERLEAVED ? (nchunks + P.q - 1) / P.q - 1 : nchunks - P.q;
-        const int rows = min(TM, P.M - m0), total = rows * ncol;
+      if (last_part) __threadfence();
+      const int slots = INTERLEAVED ? arrivals : 1 + max(0, nchunks - P.q);
+      const int rows = min(TM, P.M - m0);
+      constexpr int V = 4;  // slots in flight
+      if (last_part && rows <= 32) {
+        // few rows (one of 48^3: 37 us, against 52 with a row per thread): elements over the threads
+        constexpr int U = 4;
         const float* slab0 = P.slab + (int64_t)(tile - P.whole) * P.slots * TN * TM;
-        float* c0p = C + (int64_t)m0 * P.ldc + P.coff[cls] + n0;
-        constexpr int U = 4;  // elements of a thread in flight
+        const int total = rows * ncol;
         for (int e = (int)threadIdx.x - 64; e < total; e += U * kEpiThreads) {
           float v[U];
-          float* at[U];
-          const float* from[U];
+          int at[U];
 #pragma unroll
           for (int u = 0; u < U; ++u) {
-            const int i = min(e + u * kEpiThreads, total - 1), col = i / rows, r = i - col * rows;
-            at[u] = c0p + (int64_t)r * P.ldc + col;
-            from[u] = slab0 + col * TM + r;
-            v[u] = __ldcg(at[u]);
+            const int i = min(e + u * kEpiThreads, total - 1), col = i / rows;
+            at[u] = col * TM + i - col * rows;
+            v[u] = __ldcg(slab0 + at[u]);
           }
-#pragma unroll 4
-          for (int k = 0; k < slots; ++k)
+#pragma unroll V
+          for (int k = 1; k < slots; ++k)
 #pragma unroll
-            for (int u = 0; u < U; ++u) v[u] += __ldcg(from[u] + (int64_t)k * TN * TM);
+            for (int u = 0; u < U; ++u) v[u] += __ldcg(slab0 + (int64_t)k * TN * TM + at[u]);
 #pragma unroll
           for (int u = 0; u < U; ++u)
-            if (e + u * kEpiThreads < total) *at[u] = v[u];
+            if (e + u * kEpiThreads < total)
+              C[(int64_t)(m0 + at[u] % TM) * P.ldc + P.coff[cls] + n0 + at[u] / TM] = v[u];
+        }
+      } else if (last_part && valid) {
+        // a row per thread, so that a warp reads 32 rows of a column together
+        constexpr int U = 16;  // columns in flight
+        for (int t = 0; t < w; t += U) {
+          float v[U];
+#pragma unroll
+          for (int u = 0; u < U; ++u) v[u] = t + u < w ? __ldcg(slab + (t + u) * TM) : 0.f;
+          for (int k = 1; k < slots; k += V) {
+            float x[V][U];
+#pragma unroll
+            for (int j = 0; j < V; ++j)
+#pragma unroll
+              for (int u = 0; u < U; ++u)
+                x[j][u] = k + j < slots && t + u < w ? __ldcg(slab + ((int64_t)(k + j) * TN + t + u) * TM) : 0.f;
+#pragma unroll
+            for (int j = 0; j < V; ++j)
+              if (k + j < slots)
+#pragma unroll
+                for (int u = 0; u < U; ++u) v[u] += x[j][u];
+          }
+#pragma unroll
+          for (int u = 0; u < U; ++u)
+            if (t + u < w) crow[t + u] = v[u];
         }
       }
     }
@@ -461,10 +482,10 @@ struct GemmPlan {
 };
 
 // Tiles beyond the whole rounds of the SMs are cut into parts of q chunks; q minimises the rounds
-// times their length (a quarter chunk for a unit's start and end) plus the slabs' way to memory and
-// back (about 18 us a chunk and 6.5 GB/ms).  One batch block of 48^3 (16 tiles of 5 chunks) runs as
-// 80 units instead of 16, 100 subtomograms of 96^3 (117 tiles of 40) as 585 instead of 117.
-// The interleaved order is for a basis larger than L2 (126 MB); see the top.
+// times their length (a chunk's loads at the 110 GB/s an SM takes in, 5 us for a unit's start and
+// end), the adding of the slots and the slabs' way to memory and back.  One batch block of 48^3 (16
+// tiles of 5 chunks) runs as 80 units instead of 16, 100 subtomograms of 96^3 (117 tiles of 40) as
+// 585 instead of 117.  The interleaved order is for a basis larger than L2 (126 MB); see the top.
 GemmPlan gemm_plan(const FleTc* t, int mt) {
   GemmPlan p;
   const int KB = t->Kpad / TK;
@@ -483,14 +504,17 @@ GemmPlan gemm_plan(const FleTc* t, int mt) {
   p.parts = 1;
   p.q = nchunks;
   p.slots = 0;
+  int tn = 16;
+  for (int k = 0; k < 8; ++k) tn = t->nt[k] && t->tn[k] > tn ? t->tn[k] : tn;
+  const double chunk = (p.interleaved ? 40 : 60) * (A_TILE + 128.0 * tn) / 110e3;  // us
   double best = 1e30;
   for (int q = nchunks; q >= 1 && rest > 0; --q) {
     const int parts = (nchunks + q - 1) / q;
-    const int slots = parts == 1 ? 0 : (p.interleaved ? parts - 1 : nchunks - q);
+    const int slots = parts == 1 ? 0 : (p.interleaved ? parts : 1 + nchunks - q);
     const size_t bytes = (size_t)rest * slots * TN * TM * sizeof(float);
     if (bytes > kSlabCap) continue;
     const int rounds = (rest * parts + kSMs - 1) / kSMs;
-    const double cost = rounds * (q + 0.25) + 2.0 * bytes / 6.5e9 / 0.018;
+    const double cost = rounds * (q * chunk + 5.0) + (parts > 1 ? 6.0 + 1.5 * slots : 0.0) + 2.0 * bytes / 6.5e6;
     if (cost < best - 1e-9) {
       best = cost;
       p.parts = parts;
