@@ -512,7 +512,8 @@ extern "C" int mtb_fle_forward(mtb_fle* h, const float* vol, int B, float* coeff
     MTB_LAUNCH_CHECK();
   }
   mtb_prof_begin(st);
-  const int parts = cluster_size(B, 8);
+  int parts = cluster_size(B, 8);
+  while (parts > 1 && h->cfg.ne < 512 * parts) parts /= 2;  // 512 coefficients a CTA at least
   for (int b0 = 0; b0 < B; b0 += 65535) {  // the grid's y limit
     const int n = B - b0 < 65535 ? B - b0 : 65535;
     MTB_CUDA_TRY(launch_clusters(expand_kernel, dim3(parts, n), kET, 0, parts, st,
