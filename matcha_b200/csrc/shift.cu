@@ -42,6 +42,7 @@ struct ShiftGeom {
   int mask_r2;           // mask_full: kp^2 + ip^2 + jp^2 <= (N/2)^2
   float dftshift;        // floor(U / 2)
   float uf;
+  const float2* tw;      // e^{-2 pi i k / N}, k < N, rounded from FP64
 };
 
 __device__ __forceinline__ float2 trilinear_c(const float2* __restrict__ v, int N, float z, float y, float x) {
@@ -95,18 +96,19 @@ __device__ __forceinline__ void ldg_quad(const float4* __restrict__ p, float4& l
       : "l"(p));
 }
 
-// trilinear_c from the corner quads (same weights and summation order).
+// trilinear_c from the corner quads (same weights and summation order).  32-bit offsets: the
+// table has at most 130 x 129^2 entries of 32 bytes.
 __device__ __forceinline__ float2 trilinear_quad(const float4* __restrict__ q, int N, float z, float y, float x) {
   const float z0 = floorf(z), y0 = floorf(y), x0 = floorf(x);
-  const int iz = (int)z0, iy = (int)y0, ix = (int)x0;
+  const int iz = (int)z0 + 1, iy = (int)y0 + 1, ix = (int)x0 + 1;
   const float fz = z - z0, fy = y - y0, fx = x - x0;
-  const bool in = iz >= -1 && iz < N && iy >= -1 && iy < N && ix >= -1 && ix < N;
-  const int n1 = N + 1;
-  const int64_t e0 = in ? ((int64_t)(iz + 1) * n1 + (iy + 1)) * n1 + (ix + 1) : 0;
-  const int64_t e1 = e0 + (int64_t)n1 * n1;
+  const bool in = (unsigned)iz <= (unsigned)N && (unsigned)iy <= (unsigned)N && (unsigned)ix <= (unsigned)N;
+  const uint32_t n1 = N + 1;
+  const uint32_t e0 = in ? 32u * ((iz * n1 + iy) * n1 + ix) : 0u;
+  const char* at = reinterpret_cast<const char*>(q);
   float4 a0, a1, b0, b1;
-  ldg_quad(q + 2 * e0, a0, a1);
-  ldg_quad(q + 2 * e1, b0, b1);
+  ldg_quad(reinterpret_cast<const float4*>(at + e0), a0, a1);
+  ldg_quad(reinterpret_cast<const float4*>(at + (e0 + 32u * n1 * n1)), b0, b1);
   const float2 v[8] = {make_float2(a0.x, a0.y), make_float2(a0.z, a0.w), make_float2(a1.x, a1.y),
                        make_float2(a1.z, a1.w), make_float2(b0.x, b0.y), make_float2(b0.z, b0.w),
                        make_float2(b1.x, b1.y), make_float2(b1.z, b1.w)};
@@ -160,6 +162,24 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
   return s;  // valid in thread 0
 }
 
+// Both sums at once (red: 64 floats); valid in thread 0.
+__device__ __forceinline__ float2 block_sum2(float2 v, float* red) {
+  v.x = warp_sum(v.x);
+  v.y = warp_sum(v.y);
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  if (lane == 0) {
+    red[w] = v.x;
+    red[32 + w] = v.y;
+  }
+  __syncthreads();
+  float2 s = make_float2(0.f, 0.f);
+  if (threadIdx.x < 32) {
+    const bool in = threadIdx.x < (blockDim.x >> 5);
+    s = make_float2(warp_sum(in ? red[threadIdx.x] : 0.f), warp_sum(in ? red[32 + threadIdx.x] : 0.f));
+  }
+  return s;
+}
+
 // ------------------------------------------------------------------ radix-2 FFT in shared memory
 __host__ __device__ constexpr int ilog2c(int n) { return n <= 1 ? 0 : 1 + ilog2c(n >> 1); }
 
@@ -169,14 +189,11 @@ __device__ __forceinline__ int brev(int k) {
   return (int)(__brev((unsigned)k) >> kShift);
 }
 
-__device__ void load_twiddles(float2* tw, int L, int count) {
-  for (int k = threadIdx.x; k < count; k += blockDim.x) {
-    double s, c;
-    sincospi(-2.0 * k / L, &s, &c);
-    tw[k] = make_float2((float)c, (float)s);
-  }
+// Twiddles e^{-2 pi i k / N}, k < count, from the handle's table (computing them took an FP64 sincos
+// in front of every CTA's loads).
+__device__ __forceinline__ void load_twiddles(float2* tw, const ShiftGeom& g, int count) {
+  for (int k = threadIdx.x; k < count; k += blockDim.x) tw[k] = __ldg(&g.tw[k]);
 }
-
 
 // Boxes that are not powers of two (48, 80, 96) take the same kernels with the radix-2 FFTs
 // replaced by direct DFTs (O(N^2) per line, natural-order output) and the index rolls done by
@@ -301,7 +318,7 @@ patch_fft_xy_kernel(const float* __restrict__ vol, const float* __restrict__ shi
   const int ip = blockIdx.x, b = blockIdx.y;
   const int i = wrap_n<N>(ip + HN);
   const int di = i - HN;
-  load_twiddles(tw, N, NTW);
+  load_twiddles(tw, g, NTW);
   auto put = [&](int jp, int kp, float val) {
     reinterpret_cast<float*>(zb + (jp < HN ? jp : jp - HN) * N + kp)[jp >= HN ? 1 : 0] = val;
   };
@@ -387,6 +404,124 @@ constexpr size_t xy_smem_bytes() {
          (size_t)2 * N * N * sizeof(float);
 }
 
+// ------------------------------------------------------------------ product with the reference
+// The product conj(S) T only exists where the Fourier ball mask is (kp^2 + jq^2 + xq^2 <= (N/2)^2 on
+// the (N, N, N/2+1) index grid, setup_utils.py:239-249): 52 % of the grid.  So for a plane jp
+//   - columns m2 of which no point lies in the ball are not transformed along z (|T|^2, which
+//     counts them, is taken before the transform, which only scales it by N);
+//   - the reference is sampled by units of a warp along a column's points in the ball
+//     (-K <= kp <= K), and in the split layout nothing else is written: the operands start zeroed
+//     and their other entries never change.
+// The reference's gathers bound the z pass, by the L1 they go through, so that what shares it
+// counts too: a line's FFT transposes through its own column instead of a scratch (box 128: 67
+// instead of 111 KB a CTA, and with two CTAs an SM the L1 keeps 90 KB).  Box 64, 1000 subtomograms
+// 1259 -> 1124 us; box 128, 48 854 -> 552 us (783 with three CTAs an SM, which leave the L1 nothing);
+// box 48, 37 with CTF 47 -> 37 us.
+template <int N>
+__device__ __forceinline__ int ball_radius(int jp, int m2) {  // K of column (jp, m2); -1: no point in the ball
+  const int jq = jp < N / 2 ? jp : jp - N, xq = m2 < N / 2 ? m2 : m2 - (N / 2 + 1);
+  const int rem = (N / 2) * (N / 2) - jq * jq - xq * xq;
+  if (rem < 0) return -1;
+  float r;
+  asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"((float)rem + 0.5f));  // the half keeps the root off integers
+  return (int)r;
+}
+
+// Columns m2 < ball_columns(jp) have points in the ball, and so has, as xq = -1, the Nyquist column
+// (but for jq = -N/2, where it is transformed all the same).
+template <int N>
+__device__ __forceinline__ int ball_columns(int jp) { return ball_radius<N>(jp, 0) + 1 < N / 2 ? ball_radius<N>(jp, 0) + 1 : N / 2; }
+
+template <int N>
+__host__ __device__ constexpr int max_units() { return (N / 2 + 1) * ((N + 31) / 32); }
+
+// The plane's units, one code m2 * 8 + chunk each, and their number; by warp 0 (a barrier follows).
+template <int N>
+__device__ __forceinline__ void list_units(int jp, uint16_t* units, int* n_units) {
+  const int lane = threadIdx.x & 31;
+  if (threadIdx.x >= 32) return;
+  int n = 0;
+  for (int m0 = 0; m0 < N / 2 + 1; m0 += 32) {
+    const int m2 = m0 + lane;
+    const int K = m2 < N / 2 + 1 ? ball_radius<N>(jp, m2) : -1;
+    const int cnt = K < 0 ? 0 : (min(2 * K + 1, N) + 31) / 32;
+    int at = cnt;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, at, o);
+      if (lane >= o) at += v;
+    }
+    for (int q = 0; q < cnt; ++q) units[n + at - cnt + q] = (uint16_t)(m2 * 8 + q);
+    n += __shfl_sync(0xffffffffu, at, 31);
+  }
+  if (lane == 0) *n_units = n;
+}
+
+// The plane's products: t_at(ip, m2) is the transformed patch, sample(z, y, x) the reference.
+// SPLIT: the pass-1 operands of the tensor-core upsampled DFT, A1[part][(b, m2, m1)][2 m0 + c] for
+// m2 < N/2 as bf16 hi/lo pairs (a1_ws pairs per row, a1_R rows per part), and the Nyquist plane
+// m2 = N/2 to a1n in the same format (rows (b, m1)).  Otherwise P overwrites T (rows of m2, zero
+// outside the ball).  Adds |S|^2 to ss.
+template <int N, bool SPLIT, class TAt, class Sample>
+__device__ __forceinline__ void ball_products(const ShiftGeom& g, int jp, int b, const uint16_t* units, int n_units,
+                                              TAt&& t_at, Sample&& sample, const float* __restrict__ rot,
+                                              const float* __restrict__ ctf, float2* __restrict__ base,
+                                              uint32_t* __restrict__ a1, int a1_ws, int a1_R,
+                                              uint32_t* __restrict__ a1n, int a1n_R, float& ss) {
+  constexpr int HN = N / 2, H = N / 2 + 1;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  float R[9];
+#pragma unroll
+  for (int q = 0; q < 9; ++q) R[q] = __ldg(&rot[b * 9 + q]);
+  const float c = (float)g.h;  // centre of the odd-padded grid, (N+1-1)/2
+  // the product at one point of the ball, kp = ip or ip - N (index N/2 standing for -N/2)
+  const float by = (float)(jp < HN ? jp : jp - N);
+  auto product = [&](int ip, int kp, int m2) -> float2 {
+    // its offsets from the centre, after the ifftshift over (z, y) of the slice [..., N/2:] of the
+    // rotated reference
+    const float bx = (float)m2, bz = (float)kp;
+    const float rx = R[0] * bx + R[1] * by + R[2] * bz + c;
+    const float ry = R[3] * bx + R[4] * by + R[5] * bz + c;
+    const float rz = R[6] * bx + R[7] * by + R[8] * bz + c;
+    float2 s = sample(rz, ry, rx);
+    if (ctf) {
+      const float cv = __ldg(&ctf[(((int64_t)b * N + ip) * N + jp) * H + m2]);
+      s.x *= cv;
+      s.y *= cv;
+    }
+    const float2 t = t_at(ip, m2);
+    ss += s.x * s.x + s.y * s.y;
+    return make_float2(s.x * t.x + s.y * t.y, s.x * t.y - s.y * t.x);  // conj(s) * t
+  };
+  if (SPLIT) {
+#pragma unroll 2
+    for (int u = warp; u < n_units; u += warps) {
+      const int code = units[u], m2 = code >> 3, K = ball_radius<N>(jp, m2);
+      const int kp = -K + (code & 7) * 32 + lane;
+      if (kp > K || kp >= HN) continue;
+      const int ip = kp < 0 ? kp + N : kp;
+      const float2 p = product(ip, kp, m2);
+      uint32_t hi, lo;
+      split_bf16x2(p.x, p.y, hi, lo);
+      const bool nyq = m2 == HN;
+      const size_t row = nyq ? (size_t)b * N + jp : ((size_t)b * HN + m2) * N + jp;
+      uint32_t* dst = (nyq ? a1n : a1) + row * a1_ws;
+      dst[ip] = hi;
+      dst[(size_t)(nyq ? a1n_R : a1_R) * a1_ws + ip] = lo;
+    }
+  } else {
+    // a warp per row ip: its points in the ball are m2 = 0 .. K and, within -1, the Nyquist column
+    for (int ip = warp; ip < N; ip += warps) {
+      const int kp = ip < HN ? ip : ip - N, jq = jp < HN ? jp : jp - N;
+      const int rem = g.mask_r2 - kp * kp - jq * jq;
+      for (int m2 = lane; m2 < H; m2 += 32) {
+        const int xq = m2 < HN ? m2 : m2 - H;
+        base[(int64_t)ip * N * H + m2] = xq * xq <= rem ? product(ip, kp, m2) : make_float2(0.f, 0.f);
+      }
+    }
+  }
+}
+
 // ------------------------------------------------------------------ FFT along z + product
 // One CTA per (b, j').  Adds avg_b times the plane transforms of W / N^3 (what), the FFT
 // along z, then P = conj(S) T with the rotated, ifftshifted, masked Fourier reference S
@@ -400,10 +535,12 @@ fft_z_kernel(ShiftGeom g, float2* __restrict__ T, const float2* __restrict__ wha
              const float2* __restrict__ ref, const float* __restrict__ rot, const float* __restrict__ ctf,
              float* __restrict__ nrm, uint32_t* __restrict__ a1, int a1_ws, int a1_R, uint32_t* __restrict__ a1n,
              int a1n_R) {
-  constexpr int HN = N / 2, H = N / 2 + 1;
+  constexpr int H = N / 2 + 1;
   constexpr int NTW = n_twiddles<N>();
   extern __shared__ __align__(16) float2 sm2[];
-  __shared__ float red[32];
+  __shared__ float red[64];
+  __shared__ uint16_t units[max_units<N>()];
+  __shared__ int n_units;
   float2* tw = sm2;
   float2* buf = sm2 + NTW;   // N (i') x H
   float2* scr = buf + N * H; // the direct DFT's scratch (boxes that are not powers of two)
@@ -411,71 +548,27 @@ fft_z_kernel(ShiftGeom g, float2* __restrict__ T, const float2* __restrict__ wha
   float2* base = T + (int64_t)b * N * N * H + (int64_t)jp * H;
   const float2* wb = what + (int64_t)jp * H;
   const float avg = g.wsum > 0.f ? __ldg(&bg[b]) / g.wsum : 0.f;
-  load_twiddles(tw, N, NTW);
+  list_units<N>(jp, units, &n_units);
+  const int cols = ball_columns<N>(jp);
+  float st = 0.f, ss = 0.f;
+  load_twiddles(tw, g, NTW);
   for (int e = threadIdx.x; e < N * H; e += kT) {
     const int ip = e / H, m2 = e % H;
     const float2 t = base[(int64_t)ip * N * H + m2];
     const float2 w = __ldg(&wb[(int64_t)ip * N * H + m2]);
-    buf[e] = make_float2(fmaf(avg, w.x, t.x), fmaf(avg, w.y, t.y));
+    const float2 v = make_float2(fmaf(avg, w.x, t.x), fmaf(avg, w.y, t.y));
+    st += v.x * v.x + v.y * v.y;  // |T|^2 is N times that of the untransformed columns
+    if (m2 < cols || m2 == N / 2) buf[e] = v;
   }
   __syncthreads();
   transform_lines<N>(buf, scr, H, 1, H, tw);
-  float R[9];
-#pragma unroll
-  for (int q = 0; q < 9; ++q) R[q] = __ldg(&rot[b * 9 + q]);
-  const float c = (float)g.h;  // centre of the odd-padded grid, (N+1-1)/2
-  float st = 0.f, ss = 0.f;
-  for (int e = threadIdx.x; e < N * H; e += kT) {
-    // SPLIT walks m0 fastest so the bf16 rows are written contiguously
-    const int ip = SPLIT ? e % N : e / H, m2 = SPLIT ? e / N : e % H;
-    const float2 t = buf[fpos<N>(ip) * H + m2];
-    // mask_full on the (N, N, N/2+1) index grid (setup_utils.py:239-249)
-    const int kp = ip < HN ? ip : ip - N;
-    const int jq = jp < HN ? jp : jp - N;
-    const int xq = m2 < HN ? m2 : m2 - H;
-    float2 s = make_float2(0.f, 0.f);
-    if (kp * kp + jq * jq + xq * xq <= g.mask_r2) {
-      // ifftshift over (z, y) of the slice [..., N/2:] of the rotated reference
-      const int zo = wrap_n<N>(ip + HN), yo = wrap_n<N>(jp + HN), xw = m2 + HN;
-      const float bx = (float)xw - c, by = (float)yo - c, bz = (float)zo - c;
-      const float rx = R[0] * bx + R[1] * by + R[2] * bz + c;
-      const float ry = R[3] * bx + R[4] * by + R[5] * bz + c;
-      const float rz = R[6] * bx + R[7] * by + R[8] * bz + c;
-      s = trilinear_c(ref, N, rz, ry, rx);
-      if (ctf) {
-        const float cv = __ldg(&ctf[(((int64_t)b * N + ip) * N + jp) * H + m2]);
-        s.x *= cv;
-        s.y *= cv;
-      }
-    }
-    st += t.x * t.x + t.y * t.y;
-    ss += s.x * s.x + s.y * s.y;
-    // conj(s) * t
-    const float2 p = make_float2(s.x * t.x + s.y * t.y, s.x * t.y - s.y * t.x);
-    if (SPLIT) {
-      if (m2 < HN) {
-        uint32_t hi, lo;
-        split_bf16x2(p.x, p.y, hi, lo);
-        const size_t row = ((size_t)b * HN + m2) * N + jp;
-        a1[row * a1_ws + ip] = hi;
-        a1[((size_t)a1_R + row) * a1_ws + ip] = lo;
-      } else {
-        // the Nyquist plane m2 = N/2: its own pass-1 operand, rows (b, m1), K (m0, re/im)
-        uint32_t hi, lo;
-        split_bf16x2(p.x, p.y, hi, lo);
-        const size_t row = (size_t)b * N + jp;
-        a1n[row * a1_ws + ip] = hi;
-        a1n[((size_t)a1n_R + row) * a1_ws + ip] = lo;
-      }
-    } else {
-      base[(int64_t)ip * N * H + m2] = p;
-    }
-  }
-  st = block_sum(st, red);
-  ss = block_sum(ss, red);
+  ball_products<N, SPLIT>(g, jp, b, units, n_units, [&](int ip, int m2) { return buf[fpos<N>(ip) * H + m2]; },
+                          [&](float z, float y, float x) { return trilinear_c(ref, N, z, y, x); }, rot, ctf, base,
+                          a1, a1_ws, a1_R, a1n, a1n_R, ss);
+  const float2 sums = block_sum2(make_float2((float)N * st, ss), red);
   if (threadIdx.x == 0) {
-    atomicAdd(&nrm[2 * b], st);
-    atomicAdd(&nrm[2 * b + 1], ss);
+    atomicAdd(&nrm[2 * b], sums.x);
+    atomicAdd(&nrm[2 * b + 1], sums.y);
   }
 }
 
@@ -537,30 +630,37 @@ __device__ __forceinline__ void fft64_group(float2 (&v)[8], int r, float2* xs, c
 }
 
 // FFT along the rows of a 64 x 33 column buffer (element (n, col) at buf[n * kZS + col], a
-// dense row stride of 33) in place, one column per group of 8 threads; xs: 36 line scratches.
+// dense row stride of 33) in place, one column per group of 8 threads, which also transposes
+// through its column: (k1, r) at row 8 k1 + (r + k1 mod 8), so that neither its writes (8 rows
+// next to each other) nor its reads (rows 8 r + (t + r mod 8)) meet in a bank.
 // The two groups of a half-warp take columns 8 apart (group 2 i + h: column (i & 7) + 16 (i / 8)
-// + 8 h), so their 8-byte accesses r + 8 s, (r + 8 s) * 33 + col fill the 16 bank pairs once;
-// the row-wise readers of the buffer, 16 consecutive rows per half-warp, do so too.
-__device__ __forceinline__ void fft64_columns(float2* buf, float2* xs, const float2* tw) {
+// + 8 h), so their 8-byte accesses r + 8 s, (r + 8 s) * 33 + col fill the 16 bank pairs once.
+// Columns from cols on are not wanted, but for the Nyquist column 32.
+__device__ __forceinline__ void fft64_columns(float2* buf, const float2* tw, int cols) {
   const int L = threadIdx.x >> 3, r = threadIdx.x & 7;
-  // groups 33..35 shadow column 32 inside its own warp
+  // groups 33..35 follow column 32 inside its own warp and write nothing
   const int col = L < 32 ? ((L >> 1) & 7) + 16 * (L >> 4) + 8 * (L & 1) : 32;
+  if (!__any_sync(0xffffffffu, col < cols || col == 32)) return;
   float2 v[8];
+  float2* c = buf + col;
 #pragma unroll
-  for (int s = 0; s < 8; ++s) v[s] = buf[(r + 8 * s) * kZS + col];
-  fft64_group(v, r, xs + L * kXS, tw);
+  for (int s = 0; s < 8; ++s) v[s] = c[(r + 8 * s) * kZS];
+  dft8(v);
+#pragma unroll
+  for (int k1 = 1; k1 < 8; ++k1) v[k1] = cmul(v[k1], tw[r * k1]);
   __syncwarp();
   if (L < 33) {
 #pragma unroll
-    for (int k2 = 0; k2 < 8; ++k2) buf[(r + 8 * k2) * kZS + col] = v[k2];
+    for (int k1 = 0; k1 < 8; ++k1) c[(8 * k1 + ((r + k1) & 7)) * kZS] = v[k1];
   }
-}
-
-__device__ void load_twiddles64(float2* tw) {
-  for (int k = threadIdx.x; k < 64; k += blockDim.x) {
-    double s, c;
-    sincospi(-2.0 * k / 64, &s, &c);
-    tw[k] = make_float2((float)c, (float)s);
+  __syncwarp();
+#pragma unroll
+  for (int t = 0; t < 8; ++t) v[t] = c[(8 * r + ((t + r) & 7)) * kZS];
+  dft8(v);
+  __syncwarp();
+  if (L < 33) {
+#pragma unroll
+    for (int k2 = 0; k2 < 8; ++k2) c[(r + 8 * k2) * kZS] = v[k2];
   }
 }
 
@@ -595,7 +695,7 @@ patch_fft_xy64_kernel(const float* __restrict__ vol, const float* __restrict__ s
   const float z0 = floorf(z);
   const int iz = (int)z0;
   const float fz = z - z0;
-  load_twiddles64(tw);
+  load_twiddles(tw, g, 64);
   if (threadIdx.x < 2 * N) {
     const int ax = threadIdx.x / N, j = threadIdx.x % N;  // ax 0: y (index j), 1: x (index k)
     const float y = (float)j + ps.f[1 + ax];
@@ -724,89 +824,45 @@ fft_z64_kernel(ShiftGeom g, float2* __restrict__ T, const float2* __restrict__ w
                const float4* __restrict__ refq, const float* __restrict__ rot, const float* __restrict__ ctf,
                float* __restrict__ nrm, uint32_t* __restrict__ a1, int a1_ws, int a1_R, uint32_t* __restrict__ a1n,
                int a1n_R) {
-  constexpr int N = 64, HN = 32, H = 33;
+  constexpr int N = 64, H = 33;
   extern __shared__ __align__(16) float2 sm2[];
-  __shared__ float red[32];
+  __shared__ float red[64];
+  __shared__ uint16_t units[max_units<N>()];
+  __shared__ int n_units;
   float2* tw = sm2;              // 64
   float2* buf = sm2 + 64;        // 64 (i') x kZS
-  float2* xs = buf + N * kZS;    // 36 x kXS
   const int jp = blockIdx.x, b = blockIdx.y;
   float2* base = T + (int64_t)b * N * N * H + (int64_t)jp * H;
   const float2* wb = what + (int64_t)jp * H;
   const float avg = g.wsum > 0.f ? __ldg(&bg[b]) / g.wsum : 0.f;
-  load_twiddles64(tw);
+  list_units<N>(jp, units, &n_units);
+  const int cols = ball_columns<N>(jp);
+  float st = 0.f, ss = 0.f;
+  load_twiddles(tw, g, 64);
 #pragma unroll 4
   for (int e = threadIdx.x; e < N * H; e += kT64) {
     const int ip = e / H, m2 = e - (e / H) * H;
     const float2 t = base[(int64_t)ip * N * H + m2];
     const float2 w = __ldg(&wb[(int64_t)ip * N * H + m2]);
-    buf[ip * kZS + m2] = make_float2(fmaf(avg, w.x, t.x), fmaf(avg, w.y, t.y));
+    const float2 v = make_float2(fmaf(avg, w.x, t.x), fmaf(avg, w.y, t.y));
+    st += v.x * v.x + v.y * v.y;  // |T|^2 is N times that of the untransformed columns
+    if (m2 < cols || m2 == N / 2) buf[ip * kZS + m2] = v;
   }
   __syncthreads();
-  fft64_columns(buf, xs, tw);
+  fft64_columns(buf, tw, cols);
   __syncthreads();
-  float R[9];
-#pragma unroll
-  for (int q = 0; q < 9; ++q) R[q] = __ldg(&rot[b * 9 + q]);
-  const float c = (float)g.h;
-  float st = 0.f, ss = 0.f;
-#pragma unroll 2
-  for (int e = threadIdx.x; e < N * H; e += kT64) {
-    const int ip = SPLIT ? e & (N - 1) : e / H, m2 = SPLIT ? e >> 6 : e - (e / H) * H;
-    const float2 t = buf[ip * kZS + m2];
-    const int kp = ip < HN ? ip : ip - N;
-    const int jq = jp < HN ? jp : jp - N;
-    const int xq = m2 < HN ? m2 : m2 - H;
-    // outside the mask the sample is taken far outside the box, which reads zero (entry 0)
-    const bool in_mask = kp * kp + jq * jq + xq * xq <= g.mask_r2;
-    float2 s;
-    {
-      const int zo = (ip + HN) & (N - 1), yo = (jp + HN) & (N - 1), xw = m2 + HN;
-      const float bx = (float)xw - c, by = (float)yo - c, bz = (float)zo - c;
-      const float rx = R[0] * bx + R[1] * by + R[2] * bz + c;
-      const float ry = R[3] * bx + R[4] * by + R[5] * bz + c;
-      const float rz = in_mask ? R[6] * bx + R[7] * by + R[8] * bz + c : -4.f;
-      s = trilinear_quad(refq, N, rz, ry, rx);
-    }
-    if (in_mask) {
-      if (ctf) {
-        const float cv = __ldg(&ctf[(((int64_t)b * N + ip) * N + jp) * H + m2]);
-        s.x *= cv;
-        s.y *= cv;
-      }
-    }
-    st += t.x * t.x + t.y * t.y;
-    ss += s.x * s.x + s.y * s.y;
-    const float2 p = make_float2(s.x * t.x + s.y * t.y, s.x * t.y - s.y * t.x);
-    if (SPLIT) {
-      if (m2 < HN) {
-        uint32_t hi, lo;
-        split_bf16x2(p.x, p.y, hi, lo);
-        const size_t row = ((size_t)b * HN + m2) * N + jp;
-        a1[row * a1_ws + ip] = hi;
-        a1[((size_t)a1_R + row) * a1_ws + ip] = lo;
-      } else {
-        // the Nyquist plane m2 = N/2: its own pass-1 operand, rows (b, m1), K (m0, re/im)
-        uint32_t hi, lo;
-        split_bf16x2(p.x, p.y, hi, lo);
-        const size_t row = (size_t)b * N + jp;
-        a1n[row * a1_ws + ip] = hi;
-        a1n[((size_t)a1n_R + row) * a1_ws + ip] = lo;
-      }
-    } else {
-      base[(int64_t)ip * N * H + m2] = p;
-    }
-  }
-  st = block_sum(st, red);
-  ss = block_sum(ss, red);
+  ball_products<N, SPLIT>(g, jp, b, units, n_units, [&](int ip, int m2) { return buf[ip * kZS + m2]; },
+                          [&](float z, float y, float x) { return trilinear_quad(refq, N, z, y, x); }, rot, ctf, base,
+                          a1, a1_ws, a1_R, a1n, a1n_R, ss);
+  const float2 sums = block_sum2(make_float2((float)N * st, ss), red);
   if (threadIdx.x == 0) {
-    atomicAdd(&nrm[2 * b], st);
-    atomicAdd(&nrm[2 * b + 1], ss);
+    atomicAdd(&nrm[2 * b], sums.x);
+    atomicAdd(&nrm[2 * b + 1], sums.y);
   }
 }
 
 constexpr size_t z64_smem_bytes() {
-  return (size_t)64 * sizeof(float2) + (size_t)64 * kZS * sizeof(float2) + (size_t)36 * kXS * sizeof(float2);
+  return (size_t)64 * sizeof(float2) + (size_t)64 * kZS * sizeof(float2);
 }
 
 // ------------------------------------------------------------------ box 128: radix-16 x 8 path
@@ -870,11 +926,30 @@ __device__ __forceinline__ void fft128_group(float2 (&v)[16], int r, float2* xs,
   }
 }
 
-__device__ void load_twiddles128(float2* tw) {
-  for (int k = threadIdx.x; k < 128; k += blockDim.x) {
-    double s, c;
-    sincospi(-2.0 * k / 128, &s, &c);
-    tw[k] = make_float2((float)c, (float)s);
+// fft128_group with its column of the 128 x 65 buffer as the scratch (see fft64_columns); a group
+// that shadows another's column writes nothing.
+__device__ __forceinline__ void fft128_column(float2 (&v)[16], int r, float2* c, const float2* tw, bool own) {
+  dft16(v);
+#pragma unroll
+  for (int k1 = 1; k1 < 16; ++k1) v[k1] = cmul(v[k1], tw[r * k1]);
+  __syncwarp();
+  if (own) {
+#pragma unroll
+    for (int k1 = 0; k1 < 16; ++k1) c[(8 * k1 + ((r + k1) & 7)) * kZS128] = v[k1];
+  }
+  __syncwarp();
+  float2 a[8], b[8];
+#pragma unroll
+  for (int t = 0; t < 8; ++t) {
+    a[t] = c[(8 * r + ((t + r) & 7)) * kZS128];       // V_t[r]
+    b[t] = c[(64 + 8 * r + ((t + r) & 7)) * kZS128];  // V_t[r + 8]
+  }
+  dft8(a);  // X[r + 16 k2]
+  dft8(b);  // X[r + 8 + 16 k2]
+#pragma unroll
+  for (int k2 = 0; k2 < 8; ++k2) {
+    v[2 * k2] = a[k2];
+    v[2 * k2 + 1] = b[k2];
   }
 }
 
@@ -913,7 +988,7 @@ patch_fft_xy128_kernel(const float* __restrict__ vol, const float* __restrict__ 
   const float z0 = floorf(z);
   const int iz = (int)z0;
   const float fz = z - z0;
-  load_twiddles128(tw);
+  load_twiddles(tw, g, 128);
   if (threadIdx.x < 2 * N) {
     const int ax = threadIdx.x / N, j = threadIdx.x % N;  // ax 0: y (index j), 1: x (index k)
     const float y = (float)j + ps.f[1 + ax];
@@ -1038,35 +1113,41 @@ fft_z128_kernel(ShiftGeom g, float2* __restrict__ T, const float2* __restrict__ 
                 int a1n_R) {
   constexpr int N = 128, HN = 64, H = 65;
   extern __shared__ __align__(16) float2 sm2[];
-  __shared__ float red[32];
+  __shared__ float red[64];
+  __shared__ uint16_t units[max_units<N>()];
+  __shared__ int n_units;
   float2* tw = sm2;                // 128
   float2* buf = sm2 + 128;         // 128 (i') x kZS128
-  float2* xs = buf + N * kZS128;   // 36 x kXS128
   const int jp = blockIdx.x, b = blockIdx.y;
   float2* base = T + (int64_t)b * N * N * H + (int64_t)jp * H;
   const float2* wb = what + (int64_t)jp * H;
   const float avg = g.wsum > 0.f ? __ldg(&bg[b]) / g.wsum : 0.f;
-  load_twiddles128(tw);
+  list_units<N>(jp, units, &n_units);
+  const int cols = ball_columns<N>(jp);
+  float st = 0.f, ss = 0.f;
+  load_twiddles(tw, g, 128);
 #pragma unroll 4
   for (int e = threadIdx.x; e < N * H; e += kT128) {
     const int ip = e / H, m2 = e - (e / H) * H;
     const float2 t = base[(int64_t)ip * N * H + m2];
     const float2 w = __ldg(&wb[(int64_t)ip * N * H + m2]);
-    buf[ip * kZS128 + m2] = make_float2(fmaf(avg, w.x, t.x), fmaf(avg, w.y, t.y));
+    const float2 v = make_float2(fmaf(avg, w.x, t.x), fmaf(avg, w.y, t.y));
+    st += v.x * v.x + v.y * v.y;  // |T|^2 is N times that of the untransformed columns
+    if (m2 < cols || m2 == N / 2) buf[ip * kZS128 + m2] = v;
   }
   __syncthreads();
   {
     const int L = threadIdx.x >> 3, r = threadIdx.x & 7;
-    float2* gx = xs + L * kXS128;
 #pragma unroll 1
     for (int round = 0; round < 2; ++round) {
       const int idx = L + kG128 * round;
       if (idx >= 72) break;
       const int col = col128(idx);
+      if (!__any_sync(0xffffffffu, col < cols || col == HN)) continue;  // no column of the warp is wanted
       float2 v[16];
 #pragma unroll
       for (int s8 = 0; s8 < 16; ++s8) v[s8] = buf[(r + 8 * s8) * kZS128 + col];
-      fft128_group(v, r, gx, tw);
+      fft128_column(v, r, buf + col, tw, idx <= 64);
       __syncwarp();
       if (idx <= 64) {
 #pragma unroll
@@ -1075,64 +1156,18 @@ fft_z128_kernel(ShiftGeom g, float2* __restrict__ T, const float2* __restrict__ 
     }
   }
   __syncthreads();
-  float R[9];
-#pragma unroll
-  for (int q = 0; q < 9; ++q) R[q] = __ldg(&rot[b * 9 + q]);
-  const float c = (float)g.h;
-  float st = 0.f, ss = 0.f;
-#pragma unroll 4
-  for (int e = threadIdx.x; e < N * H; e += kT128) {
-    const int ip = SPLIT ? e & (N - 1) : e / H, m2 = SPLIT ? e >> 7 : e - (e / H) * H;
-    const float2 t = buf[ip * kZS128 + m2];
-    const int kp = ip < HN ? ip : ip - N;
-    const int jq = jp < HN ? jp : jp - N;
-    const int xq = m2 < HN ? m2 : m2 - H;
-    // outside the mask the sample is taken far outside the box, which reads zero (entry 0)
-    const bool in_mask = kp * kp + jq * jq + xq * xq <= g.mask_r2;
-    float2 s;
-    {
-      const int zo = (ip + HN) & (N - 1), yo = (jp + HN) & (N - 1), xw = m2 + HN;
-      const float bx = (float)xw - c, by = (float)yo - c, bz = (float)zo - c;
-      const float rx = R[0] * bx + R[1] * by + R[2] * bz + c;
-      const float ry = R[3] * bx + R[4] * by + R[5] * bz + c;
-      const float rz = in_mask ? R[6] * bx + R[7] * by + R[8] * bz + c : -4.f;
-      s = trilinear_quad(refq, N, rz, ry, rx);
-    }
-    if (in_mask && ctf) {
-      const float cv = __ldg(&ctf[(((int64_t)b * N + ip) * N + jp) * H + m2]);
-      s.x *= cv;
-      s.y *= cv;
-    }
-    st += t.x * t.x + t.y * t.y;
-    ss += s.x * s.x + s.y * s.y;
-    const float2 p = make_float2(s.x * t.x + s.y * t.y, s.x * t.y - s.y * t.x);
-    if (SPLIT) {
-      uint32_t hi, lo;
-      split_bf16x2(p.x, p.y, hi, lo);
-      if (m2 < HN) {
-        const size_t row = ((size_t)b * HN + m2) * N + jp;
-        a1[row * a1_ws + ip] = hi;
-        a1[((size_t)a1_R + row) * a1_ws + ip] = lo;
-      } else {
-        // the Nyquist plane m2 = N/2: its own pass-1 operand, rows (b, m1), K (m0, re/im)
-        const size_t row = (size_t)b * N + jp;
-        a1n[row * a1_ws + ip] = hi;
-        a1n[((size_t)a1n_R + row) * a1_ws + ip] = lo;
-      }
-    } else {
-      base[(int64_t)ip * N * H + m2] = p;
-    }
-  }
-  st = block_sum(st, red);
-  ss = block_sum(ss, red);
+  ball_products<N, SPLIT>(g, jp, b, units, n_units, [&](int ip, int m2) { return buf[ip * kZS128 + m2]; },
+                          [&](float z, float y, float x) { return trilinear_quad(refq, N, z, y, x); }, rot, ctf, base,
+                          a1, a1_ws, a1_R, a1n, a1n_R, ss);
+  const float2 sums = block_sum2(make_float2((float)N * st, ss), red);
   if (threadIdx.x == 0) {
-    atomicAdd(&nrm[2 * b], st);
-    atomicAdd(&nrm[2 * b + 1], ss);
+    atomicAdd(&nrm[2 * b], sums.x);
+    atomicAdd(&nrm[2 * b + 1], sums.y);
   }
 }
 
 constexpr size_t z128_smem_bytes() {
-  return (size_t)128 * sizeof(float2) + (size_t)128 * kZS128 * sizeof(float2) + (size_t)kG128 * kXS128 * sizeof(float2);
+  return (size_t)128 * sizeof(float2) + (size_t)128 * kZS128 * sizeof(float2);
 }
 
 // ------------------------------------------------------------------ boxes 48 and 96: radix-S x 8 path
@@ -1210,22 +1245,23 @@ __host__ __device__ constexpr int grp_xs() {  // per-group scratch: 9 S entries,
 
 // N-point forward FFT (N = 8 S) of one line by its 8 threads; v[s] = x[r + 8 s] on entry; on
 // exit o[j][k2] = X[(r + 8 j) + S k2] for the j with r + 8 j < S.  gmask: the group's lanes.
-template <int S>
-__device__ __forceinline__ void fft_grp(float2 (&v)[S], int r, unsigned gmask, float2* xs, const float2* tw,
+// slot(k1, t) is the transpose's element (k1, t) in the group's scratch (t < 8).
+template <int S, class Slot>
+__device__ __forceinline__ void fft_grp(float2 (&v)[S], int r, unsigned gmask, Slot&& slot, const float2* tw,
                                         float2 (&o)[2][8]) {
   dft_small<S>(v);  // V_r[k1]
 #pragma unroll
   for (int k1 = 1; k1 < S; ++k1) v[k1] = cmul(v[k1], tw[r * k1]);
   __syncwarp(gmask);
 #pragma unroll
-  for (int k1 = 0; k1 < S; ++k1) xs[9 * k1 + r] = v[k1];
+  for (int k1 = 0; k1 < S; ++k1) slot(k1, r) = v[k1];
   __syncwarp(gmask);
 #pragma unroll
   for (int j = 0; j < 2; ++j) {
     const int k1 = r + 8 * j;
     if (k1 < S) {
 #pragma unroll
-      for (int t = 0; t < 8; ++t) o[j][t] = xs[9 * k1 + t];  // V_t[k1]
+      for (int t = 0; t < 8; ++t) o[j][t] = slot(k1, t);  // V_t[k1]
       dft8(o[j]);
     }
   }
@@ -1260,7 +1296,7 @@ patch_fft_xy_grp_kernel(const float* __restrict__ vol, const float* __restrict__
   const float z0 = floorf(z);
   const int iz = (int)z0;
   const float fz = z - z0;
-  load_twiddles(tw, N, N);
+  load_twiddles(tw, g, N);
   if (threadIdx.x < 2 * N) {
     const int ax = threadIdx.x / N, j = threadIdx.x % N;
     const float y = (float)j + ps.f[1 + ax];
@@ -1345,7 +1381,7 @@ patch_fft_xy_grp_kernel(const float* __restrict__ vol, const float* __restrict__
     const int q = L + kGG * round;
     if (q < HN) {
       float2 o[2][8];
-      fft_grp<S>(w[round], r, gmask, gx, tw, o);
+      fft_grp<S>(w[round], r, gmask, [&](int k1, int t) -> float2& { return gx[9 * k1 + t]; }, tw, o);
 #pragma unroll
       for (int j = 0; j < 2; ++j)
         if (r + 8 * j < S) {
@@ -1371,7 +1407,7 @@ patch_fft_xy_grp_kernel(const float* __restrict__ vol, const float* __restrict__
       x[s8 + S / 2] = make_float2(0.5f * (zk.y + zm.y), -0.5f * (zk.x - zm.x));
     }
     float2 o[2][8];
-    fft_grp<S>(x, r, gmask, gx, tw, o);
+    fft_grp<S>(x, r, gmask, [&](int k1, int t) -> float2& { return gx[9 * k1 + t]; }, tw, o);
 #pragma unroll
     for (int j = 0; j < 2; ++j)
       if (r + 8 * j < S) {
@@ -1398,36 +1434,41 @@ fft_z_grp_kernel(ShiftGeom g, float2* __restrict__ T, const float2* __restrict__
                  float* __restrict__ nrm, uint32_t* __restrict__ a1, int a1_ws, int a1_R, uint32_t* __restrict__ a1n,
                  int a1n_R) {
   constexpr int S = N / 8, HN = N / 2, H = N / 2 + 1;
-  constexpr int XS = grp_xs<S>();
   extern __shared__ __align__(16) float2 sm2[];
-  __shared__ float red[32];
+  __shared__ float red[64];
+  __shared__ uint16_t units[max_units<N>()];
+  __shared__ int n_units;
   float2* tw = sm2;            // N
   float2* buf = sm2 + N;       // N (i') x H
-  float2* xs = buf + N * H;    // kGG x XS
   const int jp = blockIdx.x, b = blockIdx.y;
   float2* base = T + (int64_t)b * N * N * H + (int64_t)jp * H;
   const float2* wb = what + (int64_t)jp * H;
   const float avg = g.wsum > 0.f ? __ldg(&bg[b]) / g.wsum : 0.f;
-  load_twiddles(tw, N, N);
+  list_units<N>(jp, units, &n_units);
+  const int cols = ball_columns<N>(jp);
+  float st = 0.f, ss = 0.f;
+  load_twiddles(tw, g, N);
 #pragma unroll 4
   for (int e = threadIdx.x; e < N * H; e += kTG) {
     const int ip = e / H, m2 = e - (e / H) * H;
     const float2 t = base[(int64_t)ip * N * H + m2];
     const float2 w = __ldg(&wb[(int64_t)ip * N * H + m2]);
-    buf[ip * H + m2] = make_float2(fmaf(avg, w.x, t.x), fmaf(avg, w.y, t.y));
+    const float2 v = make_float2(fmaf(avg, w.x, t.x), fmaf(avg, w.y, t.y));
+    st += v.x * v.x + v.y * v.y;  // |T|^2 is N times that of the untransformed columns
+    if (m2 < cols || m2 == N / 2) buf[ip * H + m2] = v;
   }
   __syncthreads();
   {
     const int L = threadIdx.x >> 3, r = threadIdx.x & 7;
     const unsigned gmask = 0xFFu << (threadIdx.x & 24);
-    float2* gx = xs + L * XS;
 #pragma unroll 1
     for (int col = L; col < H; col += kGG) {
+      if (col >= cols && col != HN) continue;
       float2 x[S];
 #pragma unroll
       for (int s8 = 0; s8 < S; ++s8) x[s8] = buf[(r + 8 * s8) * H + col];
       float2 o[2][8];
-      fft_grp<S>(x, r, gmask, gx, tw, o);
+      fft_grp<S>(x, r, gmask, [&](int k1, int t) -> float2& { return buf[(8 * k1 + ((t + k1) & 7)) * H + col]; }, tw, o);
       __syncwarp(gmask);  // the group has read its column: write the transform back
 #pragma unroll
       for (int j = 0; j < 2; ++j)
@@ -1438,65 +1479,19 @@ fft_z_grp_kernel(ShiftGeom g, float2* __restrict__ T, const float2* __restrict__
     }
   }
   __syncthreads();
-  float R[9];
-#pragma unroll
-  for (int q = 0; q < 9; ++q) R[q] = __ldg(&rot[b * 9 + q]);
-  const float c = (float)g.h;
-  float st = 0.f, ss = 0.f;
-#pragma unroll 4
-  for (int e = threadIdx.x; e < N * H; e += kTG) {
-    const int ip = SPLIT ? e % N : e / H, m2 = SPLIT ? e / N : e % H;
-    const float2 t = buf[ip * H + m2];
-    const int kp = ip < HN ? ip : ip - N;
-    const int jq = jp < HN ? jp : jp - N;
-    const int xq = m2 < HN ? m2 : m2 - H;
-    // outside the mask the sample is taken far outside the box, which reads zero (entry 0)
-    const bool in_mask = kp * kp + jq * jq + xq * xq <= g.mask_r2;
-    float2 s;
-    {
-      const int zo = wrap_n<N>(ip + HN), yo = wrap_n<N>(jp + HN), xw = m2 + HN;
-      const float bx = (float)xw - c, by = (float)yo - c, bz = (float)zo - c;
-      const float rx = R[0] * bx + R[1] * by + R[2] * bz + c;
-      const float ry = R[3] * bx + R[4] * by + R[5] * bz + c;
-      const float rz = in_mask ? R[6] * bx + R[7] * by + R[8] * bz + c : -4.f;
-      s = trilinear_quad(refq, N, rz, ry, rx);
-    }
-    if (in_mask && ctf) {
-      const float cv = __ldg(&ctf[(((int64_t)b * N + ip) * N + jp) * H + m2]);
-      s.x *= cv;
-      s.y *= cv;
-    }
-    st += t.x * t.x + t.y * t.y;
-    ss += s.x * s.x + s.y * s.y;
-    const float2 p = make_float2(s.x * t.x + s.y * t.y, s.x * t.y - s.y * t.x);
-    if (SPLIT) {
-      uint32_t hi, lo;
-      split_bf16x2(p.x, p.y, hi, lo);
-      if (m2 < HN) {
-        const size_t row = ((size_t)b * HN + m2) * N + jp;
-        a1[row * a1_ws + ip] = hi;
-        a1[((size_t)a1_R + row) * a1_ws + ip] = lo;
-      } else {
-        const size_t row = (size_t)b * N + jp;
-        a1n[row * a1_ws + ip] = hi;
-        a1n[((size_t)a1n_R + row) * a1_ws + ip] = lo;
-      }
-    } else {
-      base[(int64_t)ip * N * H + m2] = p;
-    }
-  }
-  st = block_sum(st, red);
-  ss = block_sum(ss, red);
+  ball_products<N, SPLIT>(g, jp, b, units, n_units, [&](int ip, int m2) { return buf[ip * H + m2]; },
+                          [&](float z, float y, float x) { return trilinear_quad(refq, N, z, y, x); }, rot, ctf, base,
+                          a1, a1_ws, a1_R, a1n, a1n_R, ss);
+  const float2 sums = block_sum2(make_float2((float)N * st, ss), red);
   if (threadIdx.x == 0) {
-    atomicAdd(&nrm[2 * b], st);
-    atomicAdd(&nrm[2 * b + 1], ss);
+    atomicAdd(&nrm[2 * b], sums.x);
+    atomicAdd(&nrm[2 * b + 1], sums.y);
   }
 }
 
 template <int N>
 constexpr size_t z_grp_smem_bytes() {
-  return (size_t)N * sizeof(float2) + (size_t)N * (N / 2 + 1) * sizeof(float2) +
-         (size_t)kGG * grp_xs<N / 8>() * sizeof(float2);
+  return (size_t)N * sizeof(float2) + (size_t)N * (N / 2 + 1) * sizeof(float2);
 }
 
 __global__ void fill_table_kernel(ShiftGeom g, int n, float* __restrict__ tab) {
@@ -1761,6 +1756,7 @@ struct mtb_shift {
   ShiftGeom g;
   float* bgw_tab;  // background weight by integer squared radius, 0 .. 3 (N/2)^2
   float* fill_tab; // fill weight W by integer squared radius (device formula)
+  float2* tw;      // g.tw
   float2* what;    // (N, N, N/2+1) plane transforms of the fill weight W / N^3
   float2* ref;     // (N, N, N) Fourier reference, fftshifted and masked
   float4* refq;    // boxes 48, 64, 96, 128: corner quads of ref, (N + 2) (N + 1)^2 x 32 bytes
@@ -2035,7 +2031,12 @@ extern "C" int mtb_shift_create(const mtb_shift_config* cfg, mtb_shift** out) {
   const bool want_tc = cfg->precision != MTB_SHIFT_FP32 && shift_tc_fits(N, g.U) == MTB_OK;
   auto fail = [&](int code) { mtb_shift_destroy(h); return code; };
   auto alloc = [&](void** p, size_t bytes) { return cudaMalloc(p, bytes > 0 ? bytes : 4) == cudaSuccess; };
-  if (!alloc((void**)&h->bgw_tab, wtab.size() * 4) || !alloc((void**)&h->fill_tab, wtab.size() * 4) || !alloc((void**)&h->what, (size_t)N * N * g.H * 8) ||
+  std::vector<float2> twt(N);
+  for (int k = 0; k < N; ++k)
+    twt[k] = 4 * k % N ? make_float2((float)cos(-2.0 * M_PI * k / N), (float)sin(-2.0 * M_PI * k / N))
+                       : make_float2(4 * k == 0 ? 1.f : (4 * k == 2 * N ? -1.f : 0.f),
+                                     4 * k == N ? -1.f : (4 * k == 3 * N ? 1.f : 0.f));  // exact on the axes
+  if (!alloc((void**)&h->tw, (size_t)N * 8) || !alloc((void**)&h->bgw_tab, wtab.size() * 4) || !alloc((void**)&h->fill_tab, wtab.size() * 4) || !alloc((void**)&h->what, (size_t)N * N * g.H * 8) ||
       !alloc((void**)&h->ref, (size_t)N * N * N * 8) || !alloc((void**)&h->E0, e0.size() * 8) ||
       !alloc((void**)&h->E1, e0.size() * 8) || !alloc((void**)&h->E2, e2.size() * 8) ||
       !alloc((void**)&h->bg, B * 4) || !alloc((void**)&h->nrm, B * 8) ||
@@ -2048,7 +2049,9 @@ extern "C" int mtb_shift_create(const mtb_shift_config* cfg, mtb_shift** out) {
   if ((N == 48 || N == 64 || N == 96 || N == 128) &&
       !alloc((void**)&h->refq, (size_t)(N + 2) * (N + 1) * (N + 1) * 32))
     return fail(MTB_ERR_OOM);
-  if (cudaMemcpy(h->bgw_tab, wtab.data(), wtab.size() * 4, cudaMemcpyHostToDevice) != cudaSuccess ||
+  h->g.tw = h->tw;
+  if (cudaMemcpy(h->tw, twt.data(), (size_t)N * 8, cudaMemcpyHostToDevice) != cudaSuccess ||
+      cudaMemcpy(h->bgw_tab, wtab.data(), wtab.size() * 4, cudaMemcpyHostToDevice) != cudaSuccess ||
       cudaMemcpy(h->E0, e0.data(), e0.size() * 8, cudaMemcpyHostToDevice) != cudaSuccess ||
       cudaMemcpy(h->E1, e0.data(), e0.size() * 8, cudaMemcpyHostToDevice) != cudaSuccess ||
       cudaMemcpy(h->E2, e2.data(), e2.size() * 8, cudaMemcpyHostToDevice) != cudaSuccess)
@@ -2070,7 +2073,7 @@ extern "C" void mtb_shift_destroy(mtb_shift* h) {
   if (!h) return;
   mtb_shift_profile(h, 0);
   shift_tc_release(&h->tc);
-  void* ptrs[] = {h->bgw_tab, h->fill_tab, h->what, h->refq, h->ref, h->E0, h->E1, h->E2, h->bg, h->nrm, h->T, h->X1, h->pval, h->pidx};
+  void* ptrs[] = {h->tw, h->bgw_tab, h->fill_tab, h->what, h->refq, h->ref, h->E0, h->E1, h->E2, h->bg, h->nrm, h->T, h->X1, h->pval, h->pidx};
   for (void* p : ptrs) if (p) cudaFree(p);
   delete h;
 }
