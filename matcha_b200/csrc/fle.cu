@@ -242,9 +242,15 @@ expand_kernel(const float* __restrict__ C, int64_t c_ld, int ne, const int2* __r
 // sigma[b][Dindex(l, m, mp)] = (-1)^(m+mp) sum_k aT[l, -mp, k] conj(aV[b][l, -m, k])
 // One CTA per (degree l, subtomogram b), largest degrees first.  The rows mu = -l..l of the
 // template and of the subtomogram's coefficients (K = kpad[l] radial entries each, gathered
-// through kidx) are staged in shared memory with an odd row stride; each output then reads
-// two rows there: sigma[l, m, m'] = (-1)^(m+m') sum_k T[-m', k] conj(V[-m, k]).
-__global__ void __launch_bounds__(256)
+// through kidx) are staged in shared memory with an odd row stride, each row with the sign
+// (-1)^mu; each output then reads two rows there: sum_k T[-m', k] conj(V[-m, k]).
+// K is small (4.5 on average at 64^3), so instruction issue bounds it, with the operand loads, the
+// row pointers and the stores beside the products: a thread takes 4 rows x 3 columns (4 x 1 284 us, 4 x
+// 2 263, 4 x 4 276, 4 x 3 255; 1000 subtomograms of 64^3, 0.85 GB of outputs, 128 us at the copy's
+// rate), and 64 registers, for eight CTAs of 128 threads an SM, 221 us.  100 of 96^3 156 -> 101 us.
+constexpr int kSC = 3, kSigmaT = 128;
+
+__global__ void __launch_bounds__(kSigmaT, 8)
 sigma_kernel(const float2* __restrict__ aV, int64_t v_stride, const float2* __restrict__ aT, int lout,
              const int* __restrict__ kpad, const int* __restrict__ koff, const int* __restrict__ kidx,
              float2* __restrict__ sigma, int64_t s_stride) {
@@ -260,41 +266,53 @@ sigma_kernel(const float2* __restrict__ aV, int64_t v_stride, const float2* __re
   for (int e = threadIdx.x; e < w * K; e += blockDim.x) {
     const int row = e / K, k = e - (e / K) * K;
     const int idx = __ldg(&tab[e]);
-    sT[row * ks + k] = idx >= 0 ? __ldg(&aT[idx]) : make_float2(0.f, 0.f);
-    sV[row * ks + k] = idx >= 0 ? __ldg(&v[idx]) : make_float2(0.f, 0.f);
+    float2 t = idx >= 0 ? __ldg(&aT[idx]) : make_float2(0.f, 0.f);
+    float2 u = idx >= 0 ? __ldg(&v[idx]) : make_float2(0.f, 0.f);
+    if (row & 1) {  // the sign (-1)^(m+mp), row by row (changing a factor's sign changes no rounding)
+      t = make_float2(-t.x, -t.y);
+      u = make_float2(-u.x, -u.y);
+    }
+    sT[row * ks + k] = t;
+    sV[row * ks + k] = u;
   }
   __syncthreads();
   float2* out = sigma + (int64_t)b * s_stride + mtb_dsize(l - 1);
-  // a thread: one column c (m' = c - l) and four rows a = 4 aq .. 4 aq + 3 (m = a - l); the
-  // lanes of a warp take consecutive c (odd row stride: no bank conflicts) and mostly share
-  // aq (the four row reads are broadcasts), so one template read serves four products
-  const int naq = (w + 3) >> 2;
-  for (int e = threadIdx.x; e < naq * w; e += blockDim.x) {
-    const int aq = e / w, c = e - (e / w) * w;
+  // a thread: four rows a = 4 aq .. 4 aq + 3 (m = a - l) and kSC columns c, c + cs, .. (m' = c - l);
+  // the lanes of a warp take consecutive c (odd row stride: no bank conflicts) and mostly share aq
+  // (the row reads are broadcasts).  Each output sums over k in order.
+  const int naq = (w + 3) >> 2, cs = (w + kSC - 1) / kSC;
+  for (int e = threadIdx.x; e < naq * cs; e += blockDim.x) {
+    const int aq = e / cs, c = e - (e / cs) * cs;
     // row of -m' is 2l - c, row of -m is 2l - a
-    const float2* tr = sT + (2 * l - c) * ks;
+    const float2* tr[kSC];
     const float2* vr[4];
 #pragma unroll
+    for (int i = 0; i < kSC; ++i) tr[i] = sT + (2 * l - min(c + i * cs, w - 1)) * ks;
+#pragma unroll
     for (int j = 0; j < 4; ++j) vr[j] = sV + (2 * l - min(4 * aq + j, w - 1)) * ks;
-    float re[4] = {0.f, 0.f, 0.f, 0.f}, im[4] = {0.f, 0.f, 0.f, 0.f};
+    float re[kSC][4] = {}, im[kSC][4] = {};
     for (int k = 0; k < K; ++k) {
-      const float2 t = tr[k];
+      float2 u[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) u[j] = vr[j][k];
+#pragma unroll
+      for (int i = 0; i < kSC; ++i) {
+        const float2 t = tr[i][k];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          // t * conj(u)
+          re[i][j] += t.x * u[j].x + t.y * u[j].y;
+          im[i][j] += t.y * u[j].x - t.x * u[j].y;
+        }
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < kSC; ++i)
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        const float2 u = vr[j][k];
-        // t * conj(u)
-        re[j] += t.x * u.x + t.y * u.y;
-        im[j] += t.y * u.x - t.x * u.y;
+        const int a = 4 * aq + j, ci = c + i * cs;
+        if (a < w && ci < w) out[a * w + ci] = make_float2(re[i][j], im[i][j]);
       }
-    }
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int a = 4 * aq + j;
-      if (a < w) {
-        const float sgn = ((a + c) & 1) ? -1.f : 1.f;  // (-1)^(m+mp) = (-1)^(a+c-2l)
-        out[a * w + c] = make_float2(sgn * re[j], sgn * im[j]);
-      }
-    }
   }
 }
 
@@ -536,10 +554,15 @@ extern "C" int mtb_sigma_upto(mtb_fle* h, const float* coeffs, int64_t coeff_str
   MTB_ARG_CHECK(coeff_stride >= h->cfg.ne, "coefficient row shorter than ne");
   MTB_ARG_CHECK(sigma_stride >= mtb_dsize(lmax_out), "sigma row shorter than dsize(lmax_out)");
   MTB_ARG_CHECK(B <= 65535, "batch too large for one launch");
-  const size_t smem = (size_t)2 * (2 * lmax_out + 1) * (h->kmax | 1) * sizeof(float2);
+  size_t rows = 0;  // entries of a degree's rows
+  for (int l = 0; l <= lmax_out; ++l) {
+    const size_t n = (size_t)(2 * l + 1) * (h->kpad_host[l] | 1);
+    rows = n > rows ? n : rows;
+  }
+  const size_t smem = 2 * rows * sizeof(float2);
   MTB_CUDA_TRY(cudaFuncSetAttribute(sigma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   mtb_prof_begin((cudaStream_t)stream);
-  sigma_kernel<<<dim3(lmax_out + 1, B), 256, smem, (cudaStream_t)stream>>>(
+  sigma_kernel<<<dim3(lmax_out + 1, B), kSigmaT, smem, (cudaStream_t)stream>>>(
       reinterpret_cast<const float2*>(coeffs), coeff_stride, reinterpret_cast<const float2*>(tmpl), lmax_out,
       h->kpad, h->koff, h->kidx, reinterpret_cast<float2*>(sigma), sigma_stride);
   mtb_prof_end((cudaStream_t)stream, "sigma_kernel");
