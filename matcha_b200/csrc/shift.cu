@@ -671,7 +671,11 @@ __device__ __forceinline__ void fft64_columns(float2* buf, const float2* tw, int
 __device__ __forceinline__ int z_at(int q, int c) { return q * 64 + (c ^ (((q & 1) << 3) | ((q << 1) & 6))); }
 
 // patch_fft_xy_kernel<64, false> with the radix-8 x 8 FFTs; fill_tab[r2] is fill_weight(r2).
-__global__ void __launch_bounds__(kT64, 4)
+// Its phases wait for one another at barriers, so the CTAs in flight count: the plane, the x FFT's
+// output and the y FFT's output take turns in one buffer, 43 instead of 58 KB, and five CTAs fit (1000
+// subtomograms 1126 -> 1030 us, 1060 with four; 320 us for the bytes).  Fewer passes through shared
+// memory (a source row interpolated once for two output rows) do not help: 1047.
+__global__ void __launch_bounds__(kT64, 5)
 patch_fft_xy64_kernel(const float* __restrict__ vol, const float* __restrict__ shift_zyx,
                       const float* __restrict__ bgw_tab, const float* __restrict__ fill_tab, ShiftGeom g,
                       float2* __restrict__ T, float* __restrict__ bg) {
@@ -683,9 +687,9 @@ patch_fft_xy64_kernel(const float* __restrict__ vol, const float* __restrict__ s
   __shared__ int4 s_ty[N];          // row j's y taps packed (c0, c1, w0, w1): one broadcast load
   float2* tw = sm2;                                     // 64
   float* P0 = reinterpret_cast<float*>(sm2 + 64);       // the z-interpolated plane
-  float2* Z = reinterpret_cast<float2*>(P0 + N * N);    // 32 x 64 x FFT output, swizzled (z_at)
-  float2* yb = reinterpret_cast<float2*>(P0);           // 64 x kYS, after the patch is built
-  float2* zb = Z + HN * N;                              // 36 x kXS: packed rows, then scratch
+  float2* Z = reinterpret_cast<float2*>(P0);            // 32 x 64 x FFT output, swizzled (z_at), over the plane
+  float2* yb = Z;                                       // 64 x kYS, over Z once it is read
+  float2* zb = Z + N * kYS;                             // 36 x kXS: packed rows, then scratch
   const int ip = blockIdx.x, b = blockIdx.y;
   const int i = (ip + HN) & (N - 1);
   const int di = i - HN;
@@ -813,8 +817,7 @@ patch_fft_xy64_kernel(const float* __restrict__ vol, const float* __restrict__ s
 }
 
 constexpr size_t xy64_smem_bytes() {
-  return (size_t)64 * sizeof(float2) + (size_t)64 * 64 * sizeof(float) + (size_t)32 * 64 * sizeof(float2) +
-         (size_t)36 * kXS * sizeof(float2);
+  return ((size_t)64 + (size_t)64 * kYS + (size_t)36 * kXS) * sizeof(float2);
 }
 
 // fft_z_kernel<64, SPLIT> with the radix-8 x 8 FFT.
