@@ -273,14 +273,17 @@ __device__ __forceinline__ void scan_group(const uint32_t* vr, int cb, int U, in
 
 // ------------------------------------------------------------------ pass 1
 // Rows (b, m2, m1) of A1 times E1 -> X1[u0] for the tile's rows, written as A2 rows
-// (b, u0, m2) with K (m1, re/im), bf16 hi and lo parts.
-template <bool ROWS_OUT>
+// (b, u0, m2) with K (m1, re/im), bf16 hi and lo parts.  Pass 2 where it is not fused: rows of A2
+// to A3.  The tiles past p's are those of n, the Nyquist plane's rows of its own operand A1n or
+// A2n, in the same launch: they are a thirtieth of the work, and on their own took a launch of 11 to
+// 27 us.  n's pass 2 leaves FP32 rows in yout; on its own (p without tiles) beside the fused passes.
 __global__ void __launch_bounds__(kThreads, 1)
-updft1_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, Pass1 p,
-                 uint32_t* __restrict__ out, float2* __restrict__ yout, int* __restrict__ err) {
+updft1_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapAn,
+                 const __grid_constant__ CUtensorMap mapB, Pass1 p, Pass1 n, uint32_t* __restrict__ out,
+                 uint32_t* __restrict__ out_n, float2* __restrict__ yout, int* __restrict__ err) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = align1024(smem_raw);
-  const int KB = p.KB, S = p.stages, NT = p.NT, NS = p.NS;
+  const int KB = p.KB, S = p.stages, NT = p.NT, NS = p.NS, tiles = p.tiles + n.tiles;
   const int B_BLK = NT * TK * 2;
   uint8_t* sB = smem;                    // [part][kb] B_BLK
   uint8_t* sA = smem + 2 * KB * B_BLK;   // [stage][part] A_TILE
@@ -321,7 +324,7 @@ updft1_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant
       for (int kb = 0; kb < KB; ++kb)
         tma_load_2d(sB + (part * KB + kb) * B_BLK, &mapB, kb * TK, (part * NS + cpart) * NT, &resF);
     int it = 0;
-    for (int tile = t0; tile < p.tiles && !abort_flag; tile += tstep) {
+    for (int tile = t0; tile < tiles && !abort_flag; tile += tstep) {
       for (int kb = 0; kb < KB; ++kb, ++it) {
         const int s = it % S;
         const uint32_t use = it / S;
@@ -331,9 +334,11 @@ updft1_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant
           break;
         }
         uint8_t* sa = sA + s * 2 * A_TILE;
+        const CUtensorMap* map = tile < p.tiles ? &mapA : &mapAn;
+        const int row = (tile < p.tiles ? tile : tile - p.tiles) * TM, R1 = tile < p.tiles ? p.R1 : n.R1;
         mbar_expect_tx(&full_bar[s], 2 * A_TILE);
-        tma_load_2d(sa, &mapA, kb * TK, tile * TM, &full_bar[s]);
-        tma_load_2d(sa + A_TILE, &mapA, kb * TK, p.R1 + tile * TM, &full_bar[s]);
+        tma_load_2d(sa, map, kb * TK, row, &full_bar[s]);
+        tma_load_2d(sa + A_TILE, map, kb * TK, R1 + row, &full_bar[s]);
       }
     }
   } else if (warp == 1 && lane == 0) {
@@ -343,7 +348,7 @@ updft1_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant
       abort_flag = 1;
     }
     int it = 0, tl = 0;
-    for (int tile = t0; ok && tile < p.tiles && !abort_flag; tile += tstep, ++tl) {
+    for (int tile = t0; ok && tile < tiles && !abort_flag; tile += tstep, ++tl) {
       const int buf = tl & 1;
       if (tl >= 2 && !mbar_wait(&accE[buf], ((tl >> 1) - 1) & 1)) {
         atomicCAS(err, 0, 23);
@@ -376,7 +381,7 @@ updft1_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant
     const int c0 = h ? c_mid : 0, c1 = h ? NT : c_mid;
     const int ubase = cpart * p.Us;
     int tl = 0;
-    for (int tile = t0; tile < p.tiles && !abort_flag; tile += tstep, ++tl) {
+    for (int tile = t0; tile < tiles && !abort_flag; tile += tstep, ++tl) {
       const int buf = tl & 1;
       if (!mbar_wait(&accF[buf], (tl >> 1) & 1)) {
         atomicCAS(err, 0, 25);
@@ -384,10 +389,11 @@ updft1_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant
         break;
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const int g = tile * TM + q * 32 + lane;
-      const bool valid = g < p.rows;
+      const bool of_n = tile >= p.tiles;
+      const int g = (of_n ? tile - p.tiles : tile) * TM + q * 32 + lane;
+      const bool valid = g < (of_n ? n.rows : p.rows);
       const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * 256);
-      if (ROWS_OUT) {
+      if (of_n && yout) {
         // row g of the product as FP32 complex values, columns (u, re/im) -> yout[g][u]
         float2* yr = yout + (size_t)g * p.U;
         tmem_for_groups(taddr, c0, c1, [&](const uint32_t(&r)[16], int cb) {
@@ -399,11 +405,15 @@ updft1_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant
           }
         });
       } else {
-        const int b = g / p.rpb, rem = g - (g / p.rpb) * p.rpb;
-        const int x = rem / p.Y, y = rem - (rem / p.Y) * p.Y;
-        const size_t row0 = (size_t)b * p.SB + (size_t)x * p.SX;  // + u * SU
+        const int rpb = of_n ? n.rpb : p.rpb, Y = of_n ? n.Y : p.Y;
+        const int b = g / rpb, rem = g - b * rpb;
+        const int x = rem / Y, y = rem - x * Y;
+        const size_t row0 = (size_t)b * (of_n ? n.SB : p.SB) + (size_t)x * (of_n ? n.SX : p.SX);  // + u * SU
+        const int SU = of_n ? n.SU : p.SU;
+        const size_t ws = of_n ? n.ws : p.ws, Rout = of_n ? n.Rout : p.Rout;
+        uint32_t* to = of_n ? out_n : out;
         tmem_for_groups(taddr, c0, c1, [&](const uint32_t(&r)[16], int cb) {
-          epi1_group<16>(r, cb, valid, ubase, p.Us, p.U, row0, p.SU, (size_t)p.ws, y, (size_t)p.Rout, out);
+          epi1_group<16>(r, cb, valid, ubase, p.Us, p.U, row0, SU, ws, y, Rout, to);
         });
       }
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -1151,42 +1161,22 @@ Pass1 pass1_params(const ShiftTc* t, int rows, int R1) {
   return p;
 }
 
-int pass1_grid(const ShiftTc* t, const Pass1& p) {
-  const int per = t->n_sm / p.NS > 0 ? t->n_sm / p.NS : 1;
-  return (p.tiles < per ? p.tiles : per) * p.NS;
+int pass1_grid(const ShiftTc* t, int tiles, int NS) {
+  const int per = t->n_sm / NS > 0 ? t->n_sm / NS : 1;
+  return (tiles < per ? tiles : per) * NS;
 }
 }  // namespace
 
 int shift_tc_passes(ShiftTc* t, int B, cudaStream_t st, const cudaEvent_t* marks) {
   MTB_CUDA_TRY(cudaMemsetAsync(t->best, 0, (size_t)B * 8, st));
   const int N = t->N, U = t->U, HH = t->HH;
-  MTB_CUDA_TRY(cudaFuncSetAttribute(updft1_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)t->smem1));
-  MTB_CUDA_TRY(cudaFuncSetAttribute(updft1_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)t->smem1));
+  MTB_CUDA_TRY(cudaFuncSetAttribute(updft1_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)t->smem1));
   const CUtensorMap& mapE1 = *reinterpret_cast<const CUtensorMap*>(t->mapE1);
-  // Nyquist plane: pass 1 over its rows (b, m1) into A2n rows (b, u0), then A2n E1 -> Y
-  {
-    Pass1 pn = pass1_params(t, B * N, t->R1n);
-    pn.rpb = N;  // row (b, m1) -> A2n row b U + u0, word m1
-    pn.Y = N;
-    pn.SB = U;
-    pn.SU = 1;
-    pn.Rout = t->R2n;
-    mtb_prof_begin(st);
-    updft1_tc_kernel<false><<<pass1_grid(t, pn), kThreads, t->smem1, st>>>(
-        *reinterpret_cast<const CUtensorMap*>(t->mapA1n), mapE1, pn, (uint32_t*)t->A2n, nullptr, t->err);
-    mtb_prof_end(st, "updft1_tc_kernel (Nyquist plane, pass 1)");
-    MTB_LAUNCH_CHECK();
-    Pass1 py = pass1_params(t, B * U, t->R2n);  // the A operand is now A2n
-    mtb_prof_begin(st);
-    updft1_tc_kernel<true><<<pass1_grid(t, py), kThreads, t->smem1, st>>>(
-        *reinterpret_cast<const CUtensorMap*>(t->mapA2n), mapE1, py, nullptr, t->nyq, t->err);
-    mtb_prof_end(st, "updft1_tc_kernel (Nyquist plane, pass 2)");
-    MTB_LAUNCH_CHECK();
-  }
+  const CUtensorMap& mapA1n = *reinterpret_cast<const CUtensorMap*>(t->mapA1n);
+  const CUtensorMap& mapA2n = *reinterpret_cast<const CUtensorMap*>(t->mapA2n);
   if (marks && marks[0]) cudaEventRecord(marks[0], st);
-  // pass 1: row (b, m2, m1) -> A2 row (b U + u0) HH + m2, word m1
+  // pass 1: row (b, m2, m1) -> A2 row (b U + u0) HH + m2, word m1, and the Nyquist plane's row
+  // (b, m1) -> A2n row b U + u0, word m1
   Pass1 p1 = pass1_params(t, B * HH * N, t->R1);
   p1.rpb = HH * N;
   p1.Y = N;
@@ -1194,11 +1184,29 @@ int shift_tc_passes(ShiftTc* t, int B, cudaStream_t st, const cudaEvent_t* marks
   p1.SX = 1;
   p1.SU = HH;
   p1.Rout = t->R2;
+  Pass1 pn = pass1_params(t, B * N, t->R1n);
+  pn.rpb = N;
+  pn.Y = N;
+  pn.SB = U;
+  pn.SU = 1;
+  pn.Rout = t->R2n;
   mtb_prof_begin(st);
-  updft1_tc_kernel<false><<<pass1_grid(t, p1), kThreads, t->smem1, st>>>(
-      *reinterpret_cast<const CUtensorMap*>(t->mapA1), mapE1, p1, (uint32_t*)t->A2, nullptr, t->err);
+  updft1_tc_kernel<<<pass1_grid(t, p1.tiles + pn.tiles, p1.NS), kThreads, t->smem1, st>>>(
+      *reinterpret_cast<const CUtensorMap*>(t->mapA1), mapA1n, mapE1, p1, pn, (uint32_t*)t->A2, (uint32_t*)t->A2n,
+      nullptr, t->err);
   mtb_prof_end(st, "updft1_tc_kernel");
   MTB_LAUNCH_CHECK();
+  // the Nyquist plane's pass 2, A2n E1 -> Y, in pass 2's launch or on its own beside the fused passes
+  const Pass1 py = pass1_params(t, B * U, t->R2n);
+  if (t->fused) {
+    Pass1 none = py;
+    none.tiles = 0;
+    mtb_prof_begin(st);
+    updft1_tc_kernel<<<pass1_grid(t, py.tiles, py.NS), kThreads, t->smem1, st>>>(
+        mapA2n, mapA2n, mapE1, none, py, nullptr, nullptr, t->nyq, t->err);
+    mtb_prof_end(st, "updft1_tc_kernel (Nyquist plane, pass 2)");
+    MTB_LAUNCH_CHECK();
+  }
   if (marks && marks[1]) cudaEventRecord(marks[1], st);
   if (!t->fused) {
     // pass 2: row (b, u0, m2) -> A3 row b RP3 + u0 U + u1, word m2
@@ -1211,8 +1219,9 @@ int shift_tc_passes(ShiftTc* t, int B, cudaStream_t st, const cudaEvent_t* marks
     p2.ws = t->KB3 * (TK / 2);
     p2.Rout = t->R3;
     mtb_prof_begin(st);
-    updft1_tc_kernel<false><<<pass1_grid(t, p2), kThreads, t->smem1, st>>>(
-        *reinterpret_cast<const CUtensorMap*>(t->mapA2), mapE1, p2, (uint32_t*)t->A3, nullptr, t->err);
+    updft1_tc_kernel<<<pass1_grid(t, p2.tiles + py.tiles, p2.NS), kThreads, t->smem1, st>>>(
+        *reinterpret_cast<const CUtensorMap*>(t->mapA2), mapA2n, mapE1, p2, py, (uint32_t*)t->A3, nullptr, t->nyq,
+        t->err);
     mtb_prof_end(st, "updft1_tc_kernel (pass 2)");
     MTB_LAUNCH_CHECK();
     Pass3 p3;
