@@ -10,12 +10,15 @@
 //   interleaved  a stage holds the hi and lo tiles of both operands, 32 along K, for all three
 //                products: the same bytes per stage, two thirds of the bytes per product, and B_hi
 //                read once instead of twice.  (With stages of 64 along K only two fit, which was
-//                1242 against 1187 us on the second line below and 2.2x slower on the first.)
-// The second is for a basis that does not stay in L2 (64^3 up: 500 MB), where the loads, into
-// shared memory and from DRAM, set the pace; below, where the whole GEMM takes tens of us, the
-// first.  Times of the GEMM, before (segmented, one CTA per tile) and now: 1000 subtomograms of
-// 64^3 679 -> 550 us (1.46 PFLOP/s issued), 100 of 96^3 1397 -> 1105 us (5.5 TB/s of basis), 256 of
-// 64^3 321 -> 177 us, one of 64^3 291 -> 102 us, 128 of 48^3 138 -> 66 us, one of 48^3 118 -> 38 us.
+//                1242 against 1187 us for 100 of 96^3 and 2.2x slower for 1000 of 64^3.)
+// The second is for a basis past 1 GB (80^3: 2 GB), where the loads, into shared memory and from
+// DRAM, set the pace.  Below, the first: it adds the same chunks in the same order however the tiles
+// are cut, so that the coefficients keep their bits, and with them the orientation search its
+// choice between equal scores (the angles at beta = 0, alpha at 0 or 2 pi), which any rounding
+// moves; at 64^3 (500 MB) the second would save 15 to 30 % of the GEMM (1000 subtomograms 550
+// against 648 us).  Times of the GEMM, before (segmented, one CTA per tile) and now: 100 of 96^3
+// 1397 -> 1105 us (5.5 TB/s of basis), 128 of 80^3 647 -> 381 us, 1000 of 64^3 679 -> 648 us, 256 of
+// 64^3 321 -> 237 us, one of 64^3 291 -> 144 us, 128 of 48^3 138 -> 66 us, one of 48^3 118 -> 38 us.
 //
 // Accumulation: the tensor core adds each K=16 product into the FP32 accumulator with a
 // truncating alignment, an error of about one unit in the last place of the accumulator per
@@ -474,6 +477,7 @@ int make_map(CUtensorMap* map, void* base, uint64_t inner, uint64_t rows, uint32
 
 constexpr int kSMs = 148;
 constexpr size_t kSlabCap = (size_t)128 << 20;  // bytes of slabs a plan may take
+constexpr size_t kInterleaveBytes = (size_t)1 << 30;  // see the top
 
 // How a GEMM of mt batch blocks is cut into units.
 struct GemmPlan {
@@ -485,7 +489,7 @@ struct GemmPlan {
 // times their length (a chunk's loads at the 110 GB/s an SM takes in, 5 us for a unit's start and
 // end), the adding of the slots and the slabs' way to memory and back.  One batch block of 48^3 (16
 // tiles of 5 chunks) runs as 80 units instead of 16, 100 subtomograms of 96^3 (117 tiles of 40) as
-// 585 instead of 117.  The interleaved order is for a basis larger than L2 (126 MB); see the top.
+// 585 instead of 117.  The interleaved order is for a basis past kInterleaveBytes; see the top.
 GemmPlan gemm_plan(const FleTc* t, int mt) {
   GemmPlan p;
   const int KB = t->Kpad / TK;
@@ -496,7 +500,7 @@ GemmPlan gemm_plan(const FleTc* t, int mt) {
     cols += t->ncols[k];
   }
   const bool all_split = t->n_split_tiles == t->n_tiles;
-  p.interleaved = all_split && cols * t->Kpad * 4 > ((size_t)126 << 20);
+  p.interleaved = all_split && cols * t->Kpad * 4 > kInterleaveBytes;
   const int nchunks = (KB * 12 + kChunkMma - 1) / kChunkMma;
   p.tiles = nt * mt;
   p.whole = p.tiles / kSMs * kSMs;
