@@ -478,7 +478,7 @@ extern "C" int mtb_sigma_backward_template(mtb_fle* h, const float* coeffs, int6
   while (n_sub > 1 && n_sub * rows + rows / 2 > 200 * 1024) --n_sub;
   const size_t smem = n_sub * rows + rows / 2;  // and a gather index for each entry
   MTB_CUDA_TRY(cudaFuncSetAttribute(sigma_backward_template_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)smem));
+                                    200 * 1024));
   mtb_prof_begin(st);
   sigma_backward_template_kernel<<<dim3(kBR, (w + kBC - 1) / kBC, lmax_g + 1), kBT, smem, st>>>(
       reinterpret_cast<const float2*>(coeffs), coeff_stride, reinterpret_cast<const float2*>(grad_sigma), grad_stride,

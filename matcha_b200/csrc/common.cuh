@@ -26,6 +26,12 @@
 
 void mtb_set_last_error(const char* msg, const char* file, int line);
 
+// Shared memory a CTA may opt in to, dynamic and static together.  A kernel's limit on its dynamic
+// part (cudaFuncAttributeMaxDynamicSharedMemorySize) belongs to the kernel, not to a launch, so a
+// launch whose size depends on the handle sets a constant: with its own size, another thread's
+// smaller handle could lower the limit between this one's call and its launch, which is then refused.
+constexpr int kSmemOptIn = 227 * 1024;
+
 // Launch timing (mtb_profile_start): an event before and one after a kernel launch on its
 // stream, a no-op while recording is off.
 void mtb_prof_begin(cudaStream_t st);

@@ -560,7 +560,7 @@ extern "C" int mtb_sigma_upto(mtb_fle* h, const float* coeffs, int64_t coeff_str
     rows = n > rows ? n : rows;
   }
   const size_t smem = 2 * rows * sizeof(float2);
-  MTB_CUDA_TRY(cudaFuncSetAttribute(sigma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  MTB_CUDA_TRY(cudaFuncSetAttribute(sigma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemOptIn));
   mtb_prof_begin((cudaStream_t)stream);
   sigma_kernel<<<dim3(lmax_out + 1, B), kSigmaT, smem, (cudaStream_t)stream>>>(
       reinterpret_cast<const float2*>(coeffs), coeff_stride, reinterpret_cast<const float2*>(tmpl), lmax_out,

@@ -66,7 +66,7 @@ constexpr int kMaxStages = 8;
 constexpr int A_TILE = TM * TK * 2;  // 16 KB
 constexpr int TKI = 32;              // K of a stage in the interleaved order
 constexpr int AI_TILE = TM * TKI * 2;
-constexpr size_t kSmemCap = 227 * 1024 - 1024;  // dynamic shared memory: the opt-in limit less the
+constexpr size_t kSmemCap = kSmemOptIn - 1024;  // dynamic shared memory: the opt-in limit less the
                                                 // static barriers
 constexpr int kThreads = 320;        // warp 0: TMA, warp 1: MMA, warps 2-9: epilogue
 constexpr int kEpiThreads = 256;
@@ -666,7 +666,7 @@ int fle_tc_forward(FleTc* t, const float* vol, int64_t vol_stride, int B, const 
   P.count = t->count;
   const size_t smem = (size_t)P.stages * P.stage_bytes + 1024;
   const auto kernel = plan.interleaved ? gemm_tc_kernel<true> : gemm_tc_kernel<false>;
-  MTB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  MTB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemCap));
   mtb_prof_begin(st);
   kernel<<<plan.units, kThreads, smem, st>>>(*reinterpret_cast<const CUtensorMap*>(t->mapA[plan.interleaved]),
                                              *reinterpret_cast<const BMaps*>(t->mapB[plan.interleaved]), P, C, t->err);

@@ -273,12 +273,12 @@ int grid_launch_t(const float2* sigma, int64_t stride, int B, const float* dtab,
   mtb_prof_begin(st);
   if (grid_staged(L0, K)) {
     MTB_CUDA_TRY(cudaFuncSetAttribute(so3_grid_topk_kernel<KC, true>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGridSmemCap));
     so3_grid_topk_kernel<KC, true><<<B, kGridThreads, smem, st>>>(sigma, stride, B, dtab, L0, 2 * L0 * K,
                                                                        C, jb, a, b, g, grid);
   } else {
     MTB_CUDA_TRY(cudaFuncSetAttribute(so3_grid_topk_kernel<KC, false>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGridSmemCap));
     so3_grid_topk_kernel<KC, false><<<B, kGridThreads, smem, st>>>(sigma, stride, B, dtab, L0, 2 * L0 * K,
                                                                         C, jb, a, b, g, grid);
   }

@@ -2168,7 +2168,7 @@ extern "C" int mtb_shift_finish(mtb_shift* h, const float* rot, const float* ctf
     return MTB_OK;
   }
   const size_t sm1 = (size_t)(U * N + N * kColTile) * 8;
-  MTB_CUDA_TRY(cudaFuncSetAttribute(updft1_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm1));
+  MTB_CUDA_TRY(cudaFuncSetAttribute(updft1_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemOptIn));
   prof_mark(h, 3, st);
   mtb_prof_begin(st);
   updft1_kernel<<<dim3((N * H + kColTile - 1) / kColTile, B), kT, sm1, st>>>(g, h->T, h->E0, h->X1);
@@ -2179,7 +2179,7 @@ extern "C" int mtb_shift_finish(mtb_shift* h, const float* rot, const float* ctf
   const int stage_e = sm2_staged <= 220 * 1024;
   const size_t sm2 = stage_e ? sm2_staged : (size_t)(N * H + U * H) * 8;
   MTB_ARG_CHECK(sm2 <= 220 * 1024 && sm1 <= 220 * 1024, "upsampled region too large for shared memory");
-  MTB_CUDA_TRY(cudaFuncSetAttribute(updft23_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm2));
+  MTB_CUDA_TRY(cudaFuncSetAttribute(updft23_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
   mtb_prof_begin(st);
   updft23_kernel<<<dim3(h->ngrp, B), kT, sm2, st>>>(g, h->X1, h->E1, h->E2, h->rows_per_cta, stage_e, h->pval,
                                                     h->pidx);

@@ -57,7 +57,7 @@ constexpr int kThreads23 = 64 + kEpi + kArg;  // warps 10-17 of updft23 take the
 constexpr int kMaxSlots = 3;         // operand slots of the fused passes 2+3
 constexpr int A_TILE = TM * TK * 2;  // one 128 x 64 bf16 K-block
 constexpr int kMaxStages = 8;
-constexpr size_t kSmemCap = 227 * 1024 - 2048;  // dynamic shared memory: the opt-in limit less the
+constexpr size_t kSmemCap = kSmemOptIn - 2048;  // dynamic shared memory: the opt-in limit less the
                                                 // kernels' static barriers, with room to spare
 
 // One complex DFT pass as a GEMM: rows of A (K = (m, re/im)) times E1 -> columns (u, re/im).
@@ -1170,7 +1170,8 @@ int pass1_grid(const ShiftTc* t, int tiles, int NS) {
 int shift_tc_passes(ShiftTc* t, int B, cudaStream_t st, const cudaEvent_t* marks) {
   MTB_CUDA_TRY(cudaMemsetAsync(t->best, 0, (size_t)B * 8, st));
   const int N = t->N, U = t->U, HH = t->HH;
-  MTB_CUDA_TRY(cudaFuncSetAttribute(updft1_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)t->smem1));
+  MTB_CUDA_TRY(cudaFuncSetAttribute(updft1_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)kSmemCap));
   const CUtensorMap& mapE1 = *reinterpret_cast<const CUtensorMap*>(t->mapE1);
   const CUtensorMap& mapA1n = *reinterpret_cast<const CUtensorMap*>(t->mapA1n);
   const CUtensorMap& mapA2n = *reinterpret_cast<const CUtensorMap*>(t->mapA2n);
@@ -1232,7 +1233,8 @@ int shift_tc_passes(ShiftTc* t, int B, cudaStream_t st, const cudaEvent_t* marks
     p3.R3 = t->R3;
     p3.NT = t->NT3;
     p3.stages = t->stages3;
-    MTB_CUDA_TRY(cudaFuncSetAttribute(updft3_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)t->smem3));
+    MTB_CUDA_TRY(cudaFuncSetAttribute(updft3_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)kSmemCap));
     const int g3 = p3.tiles < t->n_sm ? p3.tiles : t->n_sm;
     mtb_prof_begin(st);
     updft3_tc_kernel<<<g3, kThreads, t->smem3, st>>>(*reinterpret_cast<const CUtensorMap*>(t->mapA3),
@@ -1258,7 +1260,8 @@ int shift_tc_passes(ShiftTc* t, int B, cudaStream_t st, const cudaEvent_t* marks
   p2.R2 = t->R2;
   p2.NT12 = t->NT12;
   p2.NT3 = t->NT3;
-  MTB_CUDA_TRY(cudaFuncSetAttribute(updft23_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)t->smem23));
+  MTB_CUDA_TRY(cudaFuncSetAttribute(updft23_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)kSmemCap));
   const int g2 = p2.tiles < t->n_sm ? p2.tiles : t->n_sm;
   mtb_prof_begin(st);
   updft23_tc_kernel<<<g2, kThreads23, t->smem23, st>>>(*reinterpret_cast<const CUtensorMap*>(t->mapA2), mapE1,
