@@ -45,6 +45,9 @@
 // the others theirs in more (one per chunk, or one per part in the interleaved order), and the
 // part that arrives last adds them in order.  With a slab per chunk the additions are
 // those of a whole tile, so a coefficient does not depend on the split, nor on the batch it is in.
+// In the interleaved order (tiles of 40 chunks at 96^3: a slab each would be 0.6 GB) a part is a group
+// of chunks whose size belongs to the basis, whatever the batch, and a whole tile adds its groups'
+// sums in the same order, so there too the batch does not matter.
 //
 // Every mbarrier wait is bounded; on expiry the kernel records an error code, stops
 // issuing, waits (bounded) for the MMAs it issued, and frees its tensor memory before
@@ -88,8 +91,10 @@ struct TcParams {
   const int* split;     // (8, ntn): 1 = hi+lo split (three products), 0 = plain BF16 (one)
   int whole;            // tiles below this are one unit each
   int parts, q;         // units of the others: parts of q chunks
+  int group;            // interleaved: chunks whose sums are formed before they meet the others'
   int slots;            // slabs of a split tile
   float* slab;          // [split tile][slot][column][row], 256 x 128 floats each
+  float* run;           // [tile that is one unit][column][row]: sums of its groups so far
   int* count;           // parts of each split tile that have arrived (zero before the launch)
 };
 
@@ -273,44 +278,71 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
 #pragma unroll
     for (int t = 0; t < TN / 2; ++t) acc[t] = 0.f;
     bool done = true;
-    for (int c = c0; c < c1; ++c) {
-      const int i = c - c0, buf = i & 1;
-      if (abort_flag || !mbar_wait_n(&acc_full[buf], (i >> 1) & 1, polls)) {
-        atomicCAS(err, 0, 3);
-        abort_flag = 1;
-        done = false;
-        break;
-      }
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * TN + h * (TN / 2));
-      const bool to_slab = !INTERLEAVED && part > 0;
-      float* out = slab + (int64_t)(1 + c - P.q) * TN * TM;
+    auto add_chunks = [&](int from, int to) {
+      for (int c = from; c < to; ++c) {
+        const int i = c - c0, buf = i & 1;
+        if (abort_flag || !mbar_wait_n(&acc_full[buf], (i >> 1) & 1, polls)) {
+          atomicCAS(err, 0, 3);
+          abort_flag = 1;
+          done = false;
+          return;
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * TN + h * (TN / 2));
+        const bool to_slab = !INTERLEAVED && part > 0;
+        float* out = slab + (int64_t)(1 + c - P.q) * TN * TM;
 #pragma unroll
-      for (int cb = 0; cb < TN / 2; cb += 32) {
-        uint32_t v[32];
-        asm volatile(
-            "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
-            "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-            : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-              "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]),
-              "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]),
-              "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]),
-              "=r"(v[30]), "=r"(v[31])
-            : "r"(taddr + (uint32_t)cb));
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        if (to_slab) {
-          if (valid) {
+        for (int cb = 0; cb < TN / 2; cb += 32) {
+          uint32_t v[32];
+          asm volatile(
+              "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
+              "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+              : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+                "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]),
+                "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]),
+                "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]),
+                "=r"(v[30]), "=r"(v[31])
+              : "r"(taddr + (uint32_t)cb));
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+          if (to_slab) {
+            if (valid) {
 #pragma unroll
-            for (int t = 0; t < 32; ++t)
-              if (h * (TN / 2) + cb + t < ncol) out[(cb + t) * TM] = __uint_as_float(v[t]);
+              for (int t = 0; t < 32; ++t)
+                if (h * (TN / 2) + cb + t < ncol) out[(cb + t) * TM] = __uint_as_float(v[t]);
+            }
+          } else {
+#pragma unroll
+            for (int t = 0; t < 32; ++t) acc[cb + t] += __uint_as_float(v[t]);
           }
-        } else {
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        mbar_arrive_cta(&acc_empty[buf]);
+      }
+    };
+    // interleaved, a whole tile of several groups: the sums of those before the current one
+    const bool grouped = INTERLEAVED && (!is_split || P.parts == 1);
+    float* run = P.run + ((int64_t)tile * TN + h * (TN / 2)) * TM + row;
+    if (grouped) {
+      const int n_cols = valid ? ncol - h * (TN / 2) : 0;
+      for (int from = c0; from < c1 && done; from += P.group) {
+        add_chunks(from, min(c1, from + P.group));
+        if (from + P.group >= c1 || !done) break;
+        // a group's end: the sums that the parts of a cut tile leave in their slots (U loads in flight)
+        constexpr int U = 16;
 #pragma unroll
-          for (int t = 0; t < 32; ++t) acc[cb + t] += __uint_as_float(v[t]);
+        for (int t = 0; t < TN / 2; t += U) {
+          float v[U];
+#pragma unroll
+          for (int u = 0; u < U; ++u) v[u] = from > c0 && t + u < n_cols ? __ldcg(run + (t + u) * TM) : 0.f;
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            if (t + u < n_cols) __stcg(run + (t + u) * TM, from > c0 ? v[u] + acc[t + u] : acc[t + u]);
+            acc[t + u] = 0.f;
+          }
         }
       }
-      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-      mbar_arrive_cta(&acc_empty[buf]);
+    } else {
+      add_chunks(c0, c1);
     }
     float* crow = C + (int64_t)(m0 + row) * P.ldc + P.coff[cls] + n0 + h * (TN / 2);
     const int w = min(TN / 2, ncol - h * (TN / 2));  // valid columns of this half (may be < 0)
@@ -318,6 +350,18 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
       const bool direct = !is_split || P.parts == 1;
       float* out = direct ? crow : slab + (int64_t)part * TN * TM;
       const int step = direct ? 1 : TM;
+      const bool more = grouped && c1 - c0 > P.group;
+      if (more) {
+        constexpr int U = 16;
+#pragma unroll
+        for (int t = 0; t < TN / 2; t += U) {
+          float v[U];
+#pragma unroll
+          for (int u = 0; u < U; ++u) v[u] = t + u < w ? __ldcg(run + (t + u) * TM) : 0.f;
+#pragma unroll
+          for (int u = 0; u < U; ++u) acc[t + u] = v[u] + acc[t + u];
+        }
+      }
 #pragma unroll
       for (int t = 0; t < TN / 2; ++t)
         if (t < w) out[t * step] = acc[t];
@@ -483,13 +527,16 @@ constexpr size_t kInterleaveBytes = (size_t)1 << 30;  // see the top
 struct GemmPlan {
   bool interleaved;
   int tiles, whole, parts, q, slots, units;
+  int runs;  // tiles that add the sums of several groups on their own
 };
 
 // Tiles beyond the whole rounds of the SMs are cut into parts of q chunks; q minimises the rounds
 // times their length (a chunk's loads at the 110 GB/s an SM takes in, 5 us for a unit's start and
 // end), the adding of the slots and the slabs' way to memory and back.  One batch block of 48^3 (16
 // tiles of 5 chunks) runs as 80 units instead of 16, 100 subtomograms of 96^3 (117 tiles of 40) as
-// 585 instead of 117.  The interleaved order is for a basis past kInterleaveBytes; see the top.
+// 585 instead of 117.  The interleaved order is for a basis past kInterleaveBytes; see the top.  There
+// the best q of one batch block is the group of every batch (t->group; 0 while it is being
+// chosen), and larger batches only choose whether to cut by it.
 GemmPlan gemm_plan(const FleTc* t, int mt) {
   GemmPlan p;
   const int KB = t->Kpad / TK;
@@ -513,6 +560,7 @@ GemmPlan gemm_plan(const FleTc* t, int mt) {
   const double chunk = (p.interleaved ? 40 : 60) * (A_TILE + 128.0 * tn) / 110e3;  // us
   double best = 1e30;
   for (int q = nchunks; q >= 1 && rest > 0; --q) {
+    if (p.interleaved && t->group && q != t->group && q != nchunks) continue;
     const int parts = (nchunks + q - 1) / q;
     const int slots = parts == 1 ? 0 : (p.interleaved ? parts : 1 + nchunks - q);
     const size_t bytes = (size_t)rest * slots * TN * TM * sizeof(float);
@@ -527,6 +575,7 @@ GemmPlan gemm_plan(const FleTc* t, int mt) {
     }
   }
   p.units = p.whole + rest * p.parts;
+  p.runs = p.interleaved && t->group < nchunks ? (p.parts == 1 ? p.tiles : p.whole) : 0;
   return p;
 }
 
@@ -603,15 +652,18 @@ int fle_tc_prepare(FleTc* t, float* const* basis, const int* class_cols, const i
       rc = make_map(reinterpret_cast<CUtensorMap*>(t->mapB[i][c]), t->B, TK, (uint64_t)rows, (uint32_t)t->tn[c], k);
   }
   if (rc) return rc;
-  // slabs and arrival counts of every batch up to max_batch
-  size_t slab = 0;
+  // slabs, running sums and arrival counts of every batch up to max_batch
+  t->group = gemm_plan(t, 1).q;
+  size_t slab = 0, run = 0;
   for (int mt = 1; mt <= t->Mpad / TM; ++mt) {
     const GemmPlan p = gemm_plan(t, mt);
+    run = p.runs > (int64_t)run ? p.runs : run;
     const size_t n = (size_t)(p.tiles - p.whole) * p.slots * TN * TM * sizeof(float);
     slab = n > slab ? n : slab;
     if (p.parts > 1 && p.tiles - p.whole > t->n_count) t->n_count = p.tiles - p.whole;
   }
   if (slab && cudaMalloc(&t->slab, slab) != cudaSuccess) return MTB_ERR_OOM;
+  if (run && cudaMalloc(&t->run, run * TN * TM * sizeof(float)) != cudaSuccess) return MTB_ERR_OOM;
   if (t->n_count && cudaMalloc(&t->count, t->n_count * sizeof(int)) != cudaSuccess) return MTB_ERR_OOM;
   return MTB_OK;
 }
@@ -622,6 +674,7 @@ void fle_tc_release(FleTc* t) {
   if (t->err) cudaFree(t->err);
   if (t->split) cudaFree(t->split);
   if (t->slab) cudaFree(t->slab);
+  if (t->run) cudaFree(t->run);
   if (t->count) cudaFree(t->count);
   memset(t, 0, sizeof(*t));
 }
@@ -661,8 +714,10 @@ int fle_tc_forward(FleTc* t, const float* vol, int64_t vol_stride, int B, const 
   P.whole = plan.whole;
   P.parts = plan.parts;
   P.q = plan.q;
+  P.group = t->group;
   P.slots = plan.slots;
   P.slab = t->slab;
+  P.run = t->run;
   P.count = t->count;
   const size_t smem = (size_t)P.stages * P.stage_bytes + 1024;
   const auto kernel = plan.interleaved ? gemm_tc_kernel<true> : gemm_tc_kernel<false>;

@@ -21,7 +21,9 @@ struct FleTc {
   int ntn;   // column tiles of the largest class
   int* split;  // (8, ntn): 1 where the tile takes the hi+lo split (three MMAs per K step), 0 where
                // its columns are all of degree <= split_degree (plain BF16, one MMA)
+  int group;    // chunks of a group (the interleaved order of the products)
   float* slab;  // partial sums of the tiles cut along K
+  float* run;   // running sums of the groups of whole tiles
   int* count;   // their parts that have arrived
   int n_count;
   int n_split_tiles, n_tiles;  // how many of the valid tiles take the split, of how many

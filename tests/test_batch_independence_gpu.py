@@ -1,0 +1,23 @@
+"""A subtomogram's results do not depend on the batch that it is sent in: every sum whose split over
+CTAs follows the batch adds the same groups in the same order.  Compared bit by bit."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("N,L,batches", [(16, 8, (1, 75, 149)), (48, 24, (1, 130, 300)), (64, 32, (1, 129, 300)), (80, 40, (1, 128, 150, 300))])
+def test_coefficients(cuda_device, N, L, batches):
+    """80^3 lies past the size from which hi and lo tiles share a stage; batches of one, two and three
+    blocks of 128, whose tiles are cut differently."""
+    from matcha_b200.core.FLEBasis3D import FLEBasis3D
+
+    cap = max(batches) + 300
+    fle = FLEBasis3D(N=N, bandlimit=L, eps=1e-4, batchsize=cap, radius=N // 2 - 1, device=cuda_device,
+                     dtype=torch.complex64, precision="bf16x3")
+    g = torch.Generator(device=cuda_device).manual_seed(N)
+    v = torch.randn((cap, N, N, N), generator=g, device=cuda_device) + 0.5
+    whole = fle._forward(v, False)[0].clone()
+    for B in batches:
+        assert torch.equal(fle._forward(v[:B], False)[0], whole[:B]), B
+    fle.status()
