@@ -186,10 +186,12 @@ gemm_fp32_kernel(const float* __restrict__ A, int64_t a_stride_class, int M, int
 // ------------------------------------------------------------------ expand + norms
 // a[b][i] = +-C[b][re_i] +- i C[b][im_i]: cols[i] holds the two columns, each shifted left by one
 // with the sign in bit 0 (-1: no imaginary part).  The work is a gather of a row that L1 holds, so
-// latency sets the time: a cluster of CTAs shares a subtomogram's coefficients, a thread has four
-// in flight, and the cluster's sums of squares meet through distributed shared memory in order.
-// 100 subtomograms of 96^3 18 us, before 111 us; one of 48^3 9 us, before 21 us (one CTA each).
-constexpr int kET = 256;
+// latency sets the time: a cluster of CTAs shares a subtomogram's coefficients and a thread has four
+// in flight.  The sum of squares is formed by `slices` of the coefficients, whose number depends on
+// ne alone and which the CTAs take in turn, so that a norm does not depend on the batch; their
+// warps' sums meet through distributed shared memory in a fixed order.  100 subtomograms of 96^3
+// 18 us, one of 48^3 9 us.
+constexpr int kET = 256, kSlices = 8;
 
 __device__ __forceinline__ float signed_at(const float* c, int code) {
   const float v = code >= 0 ? __ldg(c + (code >> 1)) : 0.f;
@@ -197,45 +199,48 @@ __device__ __forceinline__ float signed_at(const float* c, int code) {
 }
 
 __global__ void __launch_bounds__(kET)
-expand_kernel(const float* __restrict__ C, int64_t c_ld, int ne, const int2* __restrict__ cols,
+expand_kernel(const float* __restrict__ C, int64_t c_ld, int ne, int slices, const int2* __restrict__ cols,
               float2* __restrict__ out, int64_t out_stride, float* __restrict__ norms) {
   namespace cg = cooperative_groups;
   cg::cluster_group cluster = cg::this_cluster();
   const int rank = (int)cluster.block_rank(), parts = (int)cluster.num_blocks(), b = blockIdx.y;
   const float* c = C + (int64_t)b * c_ld;
   float2* o = out + (int64_t)b * out_stride;
-  float ss = 0.f;
-  const int step = parts * kET;
-  for (int i0 = rank * kET + threadIdx.x; i0 < ne; i0 += 4 * step) {
-    int2 k[4];
-    float2 v[4];
+  __shared__ float red[kSlices][kET / 32];
+  const int step = slices * kET;
+  for (int s = rank; s < slices; s += parts) {
+    float ss = 0.f;
+    for (int i0 = s * kET + threadIdx.x; i0 < ne; i0 += 4 * step) {
+      int2 k[4];
+      float2 v[4];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) k[u] = i0 + u * step < ne ? __ldg(&cols[i0 + u * step]) : make_int2(-1, -1);
+      for (int u = 0; u < 4; ++u) k[u] = i0 + u * step < ne ? __ldg(&cols[i0 + u * step]) : make_int2(-1, -1);
 #pragma unroll
-    for (int u = 0; u < 4; ++u) v[u] = make_float2(signed_at(c, k[u].x), signed_at(c, k[u].y));
+      for (int u = 0; u < 4; ++u) v[u] = make_float2(signed_at(c, k[u].x), signed_at(c, k[u].y));
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      if (i0 + u * step < ne) o[i0 + u * step] = v[u];
-      ss += v[u].x * v[u].x + v[u].y * v[u].y;
+      for (int u = 0; u < 4; ++u) {
+        if (i0 + u * step < ne) o[i0 + u * step] = v[u];
+        ss += v[u].x * v[u].x + v[u].y * v[u].y;
+      }
     }
+    ss = warp_sum(ss);
+    if ((threadIdx.x & 31) == 0) red[s][threadIdx.x >> 5] = ss;
   }
   if (!norms) return;  // the same for the whole cluster
-  __shared__ float red[kET / 32], total;
-  ss = warp_sum(ss);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    float s = 0.f;
-    for (int w = 0; w < kET / 32; ++w) s += red[w];
-    total = s;
-  }
   cluster.sync();
-  if (rank == 0 && threadIdx.x == 0) {
-    float s = 0.f;
-    for (int q = 0; q < parts; ++q) s += cluster.map_shared_rank(&total, q)[0];
-    norms[b] = sqrtf(s);
+  if (rank == 0 && threadIdx.x < 32) {
+    constexpr int kW = kET / 32, kEach = kSlices * kW / 32;  // sums of all slices' warps, kEach to a lane
+    double sum = 0.0;
+#pragma unroll
+    for (int j = 0; j < kEach; ++j) {
+      const int e = j * 32 + (int)threadIdx.x, s = e / kW;
+      if (s < slices) sum += cluster.map_shared_rank(&red[s][e % kW], s & (parts - 1))[0];
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if (threadIdx.x == 0) norms[b] = sqrtf((float)sum);
   }
-  cluster.sync();  // no CTA leaves while its sum is read
+  cluster.sync();  // no CTA leaves while its sums are read
 }
 
 // ------------------------------------------------------------------ sigma
@@ -530,13 +535,14 @@ extern "C" int mtb_fle_forward(mtb_fle* h, const float* vol, int B, float* coeff
     MTB_LAUNCH_CHECK();
   }
   mtb_prof_begin(st);
-  int parts = cluster_size(B, 8);
-  while (parts > 1 && h->cfg.ne < 512 * parts) parts /= 2;  // 512 coefficients a CTA at least
+  int slices = kSlices, parts = cluster_size(B, 8);
+  while (slices > 1 && h->cfg.ne < 512 * slices) slices /= 2;  // 512 coefficients each at least
+  parts = parts < slices ? parts : slices;
   for (int b0 = 0; b0 < B; b0 += 65535) {  // the grid's y limit
     const int n = B - b0 < 65535 ? B - b0 : 65535;
     MTB_CUDA_TRY(launch_clusters(expand_kernel, dim3(parts, n), kET, 0, parts, st,
                                  (const float*)h->C + (int64_t)b0 * h->cfg.n_cols, (int64_t)h->cfg.n_cols, h->cfg.ne,
-                                 (const int2*)h->cols, reinterpret_cast<float2*>(coeffs) + b0 * coeff_stride,
+                                 slices, (const int2*)h->cols, reinterpret_cast<float2*>(coeffs) + b0 * coeff_stride,
                                  coeff_stride, norms ? norms + b0 : nullptr));
   }
   mtb_prof_end(st, "expand_kernel");

@@ -6,7 +6,8 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("N,L,batches", [(16, 8, (1, 75, 149)), (48, 24, (1, 130, 300)), (64, 32, (1, 129, 300)), (80, 40, (1, 128, 150, 300))])
+@pytest.mark.parametrize("N,L,batches", [(16, 8, (1, 75, 149)), (48, 24, (1, 130, 300)), (64, 32, (1, 129, 300)),
+                                         (80, 40, (1, 128, 150, 300))])
 def test_coefficients(cuda_device, N, L, batches):
     """80^3 lies past the size from which hi and lo tiles share a stage; batches of one, two and three
     blocks of 128, whose tiles are cut differently."""
@@ -20,4 +21,19 @@ def test_coefficients(cuda_device, N, L, batches):
     whole = fle._forward(v, False)[0].clone()
     for B in batches:
         assert torch.equal(fle._forward(v[:B], False)[0], whole[:B]), B
+    fle.status()
+
+
+@pytest.mark.parametrize("N,L", [(16, 8), (48, 24), (64, 32)])
+def test_norms(cuda_device, N, L):
+    """Batches of every cluster size of the coefficients' sums of squares, eight CTAs to one."""
+    from matcha_b200.core.FLEBasis3D import FLEBasis3D
+
+    fle = FLEBasis3D(N=N, bandlimit=L, eps=1e-4, batchsize=1200, radius=N // 2 - 1, device=cuda_device,
+                     dtype=torch.complex64, precision="bf16x3")
+    g = torch.Generator(device=cuda_device).manual_seed(N)
+    v = (torch.randn((100, N, N, N), generator=g, device=cuda_device) + 0.5).repeat(12, 1, 1, 1)
+    whole = fle._forward(v, True)[1].clone()
+    for B in (1, 149, 297, 593):
+        assert torch.equal(fle._forward(v[:B], True)[1], whole[:B]), B
     fle.status()
