@@ -68,9 +68,8 @@ __device__ __forceinline__ Axis patch_axis(int g, float s, int N) {
   return a;
 }
 
-// Adds the block's sums of s1 and s2 to to[0] and to[1] (red: two entries per warp).
-__device__ __forceinline__ void block_add(float s1, float s2, double* to, double (&red)[2][kPT / 32]) {
-  double d1 = s1, d2 = s2;
+// Adds the block's sums of d1 and d2 to to[0] and to[1] (red: two entries per warp).
+__device__ __forceinline__ void block_add(double d1, double d2, double* to, double (&red)[2][kPT / 32]) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     d1 += __shfl_xor_sync(0xffffffffu, d1, o);
@@ -164,7 +163,7 @@ struct RowAxis {
 // Shared memory: the y axis (N entries) and one plane (N^2 floats, the z interpolation of planes
 // iz0 and iz0 + 1).
 template <int NT>
-__global__ void __launch_bounds__(kPT, NT ? 5 : 4) extract_staged_kernel(const float* __restrict__ vol, int n_rt, int planes,
+__global__ void __launch_bounds__(kPT, NT ? 5 : 4) extract_staged_kernel(const float* __restrict__ vol, int n_rt, int planes /* 1 or 2 */,
                                                                 const float* __restrict__ shift_xyz, int thresh,
                                                                 float2* __restrict__ pairs,
                                                                 double* __restrict__ stats) {
@@ -178,7 +177,9 @@ __global__ void __launch_bounds__(kPT, NT ? 5 : 4) extract_staged_kernel(const f
   const float* v = vol + (int64_t)b * NN * N;
   const float sx = shift_xyz[3 * b], sy = shift_xyz[3 * b + 1], sz = shift_xyz[3 * b + 2];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  float s1 = 0.f, s2 = 0.f;
+  // FP32 sums of the plane in hand and of the one before: they meet in FP64, so that one or two planes
+  // a CTA make no difference
+  float s1 = 0.f, s2 = 0.f, p1 = 0.f, p2 = 0.f;
   for (int y = threadIdx.x; y < N; y += kPT) {
     const Axis a = patch_axis(y, sy, N);
     s_y[y] = RowAxis{a.w0, a.w1, a.v0 ? a.j0 * N : ~(a.j0 * N), a.v1 ? a.j1 * N : ~(a.j1 * N)};
@@ -224,6 +225,9 @@ __global__ void __launch_bounds__(kPT, NT ? 5 : 4) extract_staged_kernel(const f
     __syncthreads();
     const int rows = (yhi - ylo + kPT / 32) / (kPT / 32);  // of a warp, next to each other
     const int y0 = ylo + warp * rows, y1 = y0 + rows < yhi + 1 ? y0 + rows : yhi + 1;
+    p1 = s1;
+    p2 = s2;
+    s1 = s2 = 0.f;
     // 64 columns at a time, two of a lane; the last one's pair is the next step's first
     for (int x0 = 0; x0 < N; x0 += 63) {
       const bool last = x0 + 64 >= N, two = x0 + 32 < N;
@@ -270,7 +274,7 @@ __global__ void __launch_bounds__(kPT, NT ? 5 : 4) extract_staged_kernel(const f
       if (last) break;
     }
   }
-  block_add(s1, s2, stats + 2 * b, red);
+  block_add((double)p1 + s1, (double)p2 + s2, stats + 2 * b, red);
 }
 
 // Rotation.  CTA = (2^lz_max output planes, subtomogram b); a warp takes a brick of 2^lx x 2^ly x

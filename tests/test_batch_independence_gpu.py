@@ -1,7 +1,12 @@
 """A subtomogram's results do not depend on the batch that it is sent in: every sum whose split over
-CTAs follows the batch adds the same groups in the same order.  Compared bit by bit."""
+CTAs follows the batch adds the same groups in the same order.  Compared bit by bit, but for the
+preparation, whose statistics meet by FP64 atomics in no order."""
+import numpy as np
 import pytest
 import torch
+
+from tests.helpers import haar_quaternions
+from tests.test_prepare import _prepare_gpu
 
 pytestmark = pytest.mark.gpu
 
@@ -37,3 +42,20 @@ def test_norms(cuda_device, N, L):
     for B in (1, 149, 297, 593):
         assert torch.equal(fle._forward(v[:B], True)[1], whole[:B]), B
     fle.status()
+
+
+@pytest.mark.parametrize("N,radius", [(16, 7.0), (64, 30.0), (90, 40.0)])
+def test_preparation(cuda_device, N, radius):
+    """Batches of CTAs of one plane and of two: the statistics are FP64 sums of the same FP32 sums (in
+    any order), so mean and deviation agree but for a rounding to FP32, and the values to 3e-7 of
+    the largest.  The mean far above the deviation makes any other change of the sums show."""
+    B = -(-1184 // ((N + 3) // 4))
+    rng = np.random.default_rng(N)
+    base = (rng.standard_normal((3, N, N, N)) + 200.0).astype(np.float32)
+    vols = base[np.arange(B) % 3]
+    shifts = rng.uniform(-2, 2, (3, 3)).astype(np.float32)[np.arange(B) % 3]
+    q = haar_quaternions(rng, 3)[np.arange(B) % 3]
+    got = _prepare_gpu(vols, shifts, q, radius, cuda_device)
+    for b in range(3):
+        one = _prepare_gpu(vols[b:b + 1], shifts[b:b + 1], q[b:b + 1], radius, cuda_device)
+        np.testing.assert_allclose(got[b:b + 1], one, rtol=0, atol=3e-7 * np.abs(one).max())
