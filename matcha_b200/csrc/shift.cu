@@ -474,24 +474,25 @@ __device__ __forceinline__ void ball_products(const ShiftGeom& g, int jp, int b,
 #pragma unroll
   for (int q = 0; q < 9; ++q) R[q] = __ldg(&rot[b * 9 + q]);
   const float c = (float)g.h;  // centre of the odd-padded grid, (N+1-1)/2
-  // the product at one point of the ball, kp = ip or ip - N (index N/2 standing for -N/2)
+  // the product at one point of the ball, kp = ip or ip - N (index N/2 standing for -N/2); at a point
+  // outside (in false) the sample is taken far outside the box, which reads zero (and t_at anything)
   const float by = (float)(jp < HN ? jp : jp - N);
-  auto product = [&](int ip, int kp, int m2) -> float2 {
+  auto product = [&](int ip, int kp, int m2, bool in = true) -> float2 {
     // its offsets from the centre, after the ifftshift over (z, y) of the slice [..., N/2:] of the
     // rotated reference
     const float bx = (float)m2, bz = (float)kp;
     const float rx = R[0] * bx + R[1] * by + R[2] * bz + c;
     const float ry = R[3] * bx + R[4] * by + R[5] * bz + c;
-    const float rz = R[6] * bx + R[7] * by + R[8] * bz + c;
+    const float rz = in ? R[6] * bx + R[7] * by + R[8] * bz + c : -4.f;
     float2 s = sample(rz, ry, rx);
-    if (ctf) {
+    if (ctf && in) {
       const float cv = __ldg(&ctf[(((int64_t)b * N + ip) * N + jp) * H + m2]);
       s.x *= cv;
       s.y *= cv;
     }
     const float2 t = t_at(ip, m2);
     ss += s.x * s.x + s.y * s.y;
-    return make_float2(s.x * t.x + s.y * t.y, s.x * t.y - s.y * t.x);  // conj(s) * t
+    return in ? make_float2(s.x * t.x + s.y * t.y, s.x * t.y - s.y * t.x) : make_float2(0.f, 0.f);  // conj(s) * t
   };
   if (SPLIT) {
 #pragma unroll 2
@@ -510,15 +511,19 @@ __device__ __forceinline__ void ball_products(const ShiftGeom& g, int jp, int b,
       dst[(size_t)(nyq ? a1n_R : a1_R) * a1_ws + ip] = lo;
     }
   } else {
-    // a warp per row ip: its points in the ball are m2 = 0 .. K and, within -1, the Nyquist column
-    for (int ip = warp; ip < N; ip += warps) {
-      const int kp = ip < HN ? ip : ip - N, jq = jp < HN ? jp : jp - N;
-      const int rem = g.mask_r2 - kp * kp - jq * jq;
-      for (int m2 = lane; m2 < H; m2 += 32) {
-        const int xq = m2 < HN ? m2 : m2 - H;
-        base[(int64_t)ip * N * H + m2] = xq * xq <= rem ? product(ip, kp, m2) : make_float2(0.f, 0.f);
-      }
-    }
+    // The points m2 < N/2 row after row, so that no lane idles (in rows of N/2 + 1 points a second or
+    // third round of a warp had one, and 300 of 64^3 took 412 us instead of 334), then the Nyquist
+    // column, by the threads at the other end.  The points outside the ball go the same way as the
+    // others (40 of 96^3 with CTF 242 us, with a branch around them 293), but for box 48, where the
+    // branch is the faster (400 235 us against 265).
+    const int jq = jp < HN ? jp : jp - N, left = g.mask_r2 - jq * jq;
+    auto put = [&](int ip, int m2) {
+      const int kp = ip < HN ? ip : ip - N, xq = m2 < HN ? m2 : -1;
+      const bool in = kp * kp + xq * xq <= left;
+      base[(int64_t)ip * N * H + m2] = N != 48 || in ? product(ip, kp, m2, in) : make_float2(0.f, 0.f);
+    };
+    for (int e = threadIdx.x; e < N * HN; e += blockDim.x) put(e / HN, e % HN);
+    for (int ip = blockDim.x - 1 - threadIdx.x; ip < N; ip += blockDim.x) put(ip, HN);
   }
 }
 
@@ -548,7 +553,7 @@ fft_z_kernel(ShiftGeom g, float2* __restrict__ T, const float2* __restrict__ wha
   float2* base = T + (int64_t)b * N * N * H + (int64_t)jp * H;
   const float2* wb = what + (int64_t)jp * H;
   const float avg = g.wsum > 0.f ? __ldg(&bg[b]) / g.wsum : 0.f;
-  list_units<N>(jp, units, &n_units);
+  if (SPLIT) list_units<N>(jp, units, &n_units);
   const int cols = ball_columns<N>(jp);
   float st = 0.f, ss = 0.f;
   load_twiddles(tw, g, NTW);
@@ -558,11 +563,12 @@ fft_z_kernel(ShiftGeom g, float2* __restrict__ T, const float2* __restrict__ wha
     const float2 w = __ldg(&wb[(int64_t)ip * N * H + m2]);
     const float2 v = make_float2(fmaf(avg, w.x, t.x), fmaf(avg, w.y, t.y));
     st += v.x * v.x + v.y * v.y;  // |T|^2 is N times that of the untransformed columns
-    if (m2 < cols || m2 == N / 2) buf[e] = v;
+    if (m2 < cols || m2 == N / 2) buf[ip * H + min(m2, cols)] = v;  // the Nyquist column after the others
   }
   __syncthreads();
-  transform_lines<N>(buf, scr, H, 1, H, tw);
-  ball_products<N, SPLIT>(g, jp, b, units, n_units, [&](int ip, int m2) { return buf[fpos<N>(ip) * H + m2]; },
+  transform_lines<N>(buf, scr, cols + 1, 1, H, tw);
+  ball_products<N, SPLIT>(g, jp, b, units, n_units,
+                          [&](int ip, int m2) { return buf[fpos<N>(ip) * H + min(m2, cols)]; },
                           [&](float z, float y, float x) { return trilinear_c(ref, N, z, y, x); }, rot, ctf, base,
                           a1, a1_ws, a1_R, a1n, a1n_R, ss);
   const float2 sums = block_sum2(make_float2((float)N * st, ss), red);
@@ -838,7 +844,7 @@ fft_z64_kernel(ShiftGeom g, float2* __restrict__ T, const float2* __restrict__ w
   float2* base = T + (int64_t)b * N * N * H + (int64_t)jp * H;
   const float2* wb = what + (int64_t)jp * H;
   const float avg = g.wsum > 0.f ? __ldg(&bg[b]) / g.wsum : 0.f;
-  list_units<N>(jp, units, &n_units);
+  if (SPLIT) list_units<N>(jp, units, &n_units);
   const int cols = ball_columns<N>(jp);
   float st = 0.f, ss = 0.f;
   load_twiddles(tw, g, 64);
@@ -1125,7 +1131,7 @@ fft_z128_kernel(ShiftGeom g, float2* __restrict__ T, const float2* __restrict__ 
   float2* base = T + (int64_t)b * N * N * H + (int64_t)jp * H;
   const float2* wb = what + (int64_t)jp * H;
   const float avg = g.wsum > 0.f ? __ldg(&bg[b]) / g.wsum : 0.f;
-  list_units<N>(jp, units, &n_units);
+  if (SPLIT) list_units<N>(jp, units, &n_units);
   const int cols = ball_columns<N>(jp);
   float st = 0.f, ss = 0.f;
   load_twiddles(tw, g, 128);
@@ -1447,7 +1453,7 @@ fft_z_grp_kernel(ShiftGeom g, float2* __restrict__ T, const float2* __restrict__
   float2* base = T + (int64_t)b * N * N * H + (int64_t)jp * H;
   const float2* wb = what + (int64_t)jp * H;
   const float avg = g.wsum > 0.f ? __ldg(&bg[b]) / g.wsum : 0.f;
-  list_units<N>(jp, units, &n_units);
+  if (SPLIT) list_units<N>(jp, units, &n_units);
   const int cols = ball_columns<N>(jp);
   float st = 0.f, ss = 0.f;
   load_twiddles(tw, g, N);
