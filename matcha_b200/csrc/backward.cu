@@ -197,21 +197,21 @@ score_backward_kernel(const float2* __restrict__ sigma, int64_t stride, int L, c
 // Template gradient of one degree l and kBC columns c of the sigma blocks by one cluster.
 // For fixed l the gradient is the product acc[c, k] = sum_{(b, a)} G_b[a, c] V_b[2l - a, k]
 // (signs aside) of depth B (2l + 1) and a small output (2l + 1) x K: bound by reading G once.
-// So the batch is split over the kBR CTAs of a cluster (subtomograms rank, rank + kBR, ...), the
-// columns over clusters, and inside a CTA a lane owns a column (a warp reads 32 consecutive
+// So the batch is split over the kR CTAs of a cluster (subtomograms rank, rank + kR, ...), the columns
+// over clusters, and inside a CTA a lane owns a column (a warp reads 32 consecutive
 // entries of a row of G), a warp owns kBK radial entries in registers and every n_rg-th row.
 // The partial sums meet in shared memory, then through distributed shared memory, in a fixed
 // order: deterministic, and no workspace.  The rows of V of n_sub subtomograms are gathered at a
 // time (kidx: rows mu = -l..l of kpad[l] entries, -1 padded), so a barrier covers n_sub of them.
 // 256 subtomograms at L = 32 (98 MB of G): 102 us, against 2487 us for one CTA per degree
 // that walked the batch alone.
-constexpr int kBR = 8;    // CTAs of a cluster
 constexpr int kBC = 32;   // columns
 constexpr int kBK = 8;    // radial entries of a warp
 constexpr int kBS = 4;    // subtomograms gathered at a time, where they fit
 constexpr int kBW = kBT / 32;
 
-__global__ void __cluster_dims__(kBR, 1, 1) __launch_bounds__(kBT)
+template <int kR>
+__global__ void __cluster_dims__(kR, 1, 1) __launch_bounds__(kBT)
 sigma_backward_template_kernel(const float2* __restrict__ aV, int64_t v_stride, const float2* __restrict__ gsig,
                                int64_t g_stride, int B, int lmax_g, int n_sub, int rows, const int* __restrict__ kpad,
                                const int* __restrict__ koff, const int* __restrict__ kidx,
@@ -221,7 +221,8 @@ sigma_backward_template_kernel(const float2* __restrict__ aV, int64_t v_stride, 
   int* at = reinterpret_cast<int*>(bsm + n_sub * rows);  // gather index of (a, k), its lowest bit a's parity
   namespace cg = cooperative_groups;
   cg::cluster_group cluster = cg::this_cluster();
-  const int rank = (int)cluster.block_rank();
+  const int rank = kR > 1 ? (int)cluster.block_rank() : 0;
+  auto meet = [&] { kR > 1 ? cluster.sync() : __syncthreads(); };
   const int l = lmax_g - (int)blockIdx.z;  // the widest degrees first
   const int w = 2 * l + 1, c0 = (int)blockIdx.y * kBC;
   if (c0 >= w) return;  // the same for the whole cluster
@@ -246,7 +247,7 @@ sigma_backward_template_kernel(const float2* __restrict__ aV, int64_t v_stride, 
     float2 acc[kBK];
 #pragma unroll
     for (int k = 0; k < kBK; ++k) acc[k] = make_float2(0.f, 0.f);
-    for (int b0 = rank; b0 < B; b0 += kBR * n_sub) {
+    for (int b0 = rank; b0 < B; b0 += kR * n_sub) {
       __syncthreads();
       // sV[i][a][k] = (-1)^a aV_b[l, -(a - l), k]
       for (int e = threadIdx.x; e < ne; e += kBT) {
@@ -254,7 +255,7 @@ sigma_backward_template_kernel(const float2* __restrict__ aV, int64_t v_stride, 
         float2 v[kBS];
 #pragma unroll
         for (int i = 0; i < kBS; ++i) {
-          const int b = b0 + i * kBR;
+          const int b = b0 + i * kR;
           v[i] = i < n_sub && b < B && code >= 0 ? __ldg(&aV[(int64_t)b * v_stride + (code >> 1)])
                                                  : make_float2(0.f, 0.f);
         }
@@ -265,12 +266,12 @@ sigma_backward_template_kernel(const float2* __restrict__ aV, int64_t v_stride, 
       __syncthreads();
       if (rg < nrg && c < w) {
         // rows r = (i, a) of the gathered subtomograms, eight loads in flight
-        const int have = (B - b0 + kBR - 1) / kBR, R = (have < n_sub ? have : n_sub) * w;
+        const int have = (B - b0 + kR - 1) / kR, R = (have < n_sub ? have : n_sub) * w;
         const float2* g = gsig + (int64_t)b0 * g_stride + goff + c;
         int a = rg;
         while (a >= w) {
           a -= w;
-          g += (int64_t)kBR * g_stride;
+          g += (int64_t)kR * g_stride;
         }
         for (int r = rg; r < R; r += 8 * nrg) {
           float2 gg[8];
@@ -280,7 +281,7 @@ sigma_backward_template_kernel(const float2* __restrict__ aV, int64_t v_stride, 
             a += nrg;
             while (a >= w) {
               a -= w;
-              g += (int64_t)kBR * g_stride;
+              g += (int64_t)kR * g_stride;
             }
           }
 #pragma unroll
@@ -313,23 +314,24 @@ sigma_backward_template_kernel(const float2* __restrict__ aV, int64_t v_stride, 
       }
       part[t][k][x] = s;
     }
-    cluster.sync();
-    for (int e = threadIdx.x + rank * kBT; e < nk * kBC; e += kBR * kBT) {
+    meet();
+    for (int e = threadIdx.x + rank * kBT; e < nk * kBC; e += kR * kBT) {
       const int k = e / kBC, x = e % kBC, col = c0 + x;
       if (col >= w) continue;
       const int idx = __ldg(&tab[(2 * l - col) * K + k0 + k]);
       if (idx < 0) continue;
       float2 s = make_float2(0.f, 0.f);
 #pragma unroll
-      for (int q = 0; q < kBR; ++q) {
-        const float2 u = cluster.map_shared_rank(&part[k / kBK][k % kBK][x], q)[0];
+      for (int q = 0; q < kR; ++q) {
+        const float2* from = &part[k / kBK][k % kBK][x];
+        const float2 u = kR > 1 ? cluster.map_shared_rank(from, q)[0] : *from;
         s.x += u.x;
         s.y += u.y;
       }
       if (col & 1) s = make_float2(-s.x, -s.y);
       grad_tmpl[idx] = s;
     }
-    cluster.sync();  // no CTA leaves, or overwrites its sums, while others read them
+    meet();  // no CTA leaves, or overwrites its sums, while others read them
   }
 }
 
@@ -477,10 +479,11 @@ extern "C" int mtb_sigma_backward_template(mtb_fle* h, const float* coeffs, int6
   int n_sub = kBS;
   while (n_sub > 1 && n_sub * rows + rows / 2 > 200 * 1024) --n_sub;
   const size_t smem = n_sub * rows + rows / 2;  // and a gather index for each entry
-  MTB_CUDA_TRY(cudaFuncSetAttribute(sigma_backward_template_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    200 * 1024));
+  // up to kBS subtomograms are one gather of a CTA: eight would only meet (one of 64^3 10.3 us, 13.7)
+  const auto kernel = B <= kBS ? sigma_backward_template_kernel<1> : sigma_backward_template_kernel<8>;
+  MTB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
   mtb_prof_begin(st);
-  sigma_backward_template_kernel<<<dim3(kBR, (w + kBC - 1) / kBC, lmax_g + 1), kBT, smem, st>>>(
+  kernel<<<dim3(B <= kBS ? 1 : 8, (w + kBC - 1) / kBC, lmax_g + 1), kBT, smem, st>>>(
       reinterpret_cast<const float2*>(coeffs), coeff_stride, reinterpret_cast<const float2*>(grad_sigma), grad_stride,
       B, lmax_g, n_sub, (int)(rows / sizeof(float2)), kpad, koff, kidx, reinterpret_cast<float2*>(grad_tmpl));
   mtb_prof_end(st, "sigma_backward_template_kernel");

@@ -126,3 +126,25 @@ def test_rotation_angles_and_gradient(cuda_device, B):
     assert bool((ang[1] >= 0).all())
     ref = (right_jacobian(omega).transpose(-1, -2) @ body[..., None])[..., 0]
     torch.testing.assert_close(out.cpu(), ref, atol=1e-9, rtol=0)
+
+
+@pytest.mark.parametrize("B", [2, 4, 5, 8])
+def test_template_gradient_of_few(cuda_device, B):
+    """A batch that one CTA gathers whole, and the smallest ones that a cluster shares, against the sum
+    of the subtomograms' gradients one by one (FP32 sums of a few hundred terms: 2e-6 of the largest)."""
+    from matcha_b200.autograd import template_sigma
+    from matcha_b200.core.CrossCorrelationMatcher import CrossCorrelationMatcher
+
+    g = torch.Generator(device=cuda_device).manual_seed(B)
+    cc = CrossCorrelationMatcher(N=32, device=cuda_device, batchsize=B, bandlimit=16, radius=15, precision="fp32")
+    v = torch.randn((B, 32, 32, 32), generator=g, device=cuda_device)
+    w = torch.randn((B, cc.sigma.shape[1]), generator=g, device=cuda_device, dtype=torch.complex64)
+
+    def grad(sl):
+        cc.expand(v[sl])
+        t = torch.ones((cc.fle.ne + 1,), device=cuda_device, dtype=torch.complex64, requires_grad=True)
+        template_sigma(t, cc, cc.lmax).backward(w[sl])
+        return t.grad.to(torch.complex128)
+
+    want = sum(grad(slice(b, b + 1)) for b in range(B))
+    assert (grad(slice(0, B)) - want).abs().max() < 2e-6 * want.abs().max()
