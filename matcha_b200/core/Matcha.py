@@ -183,10 +183,8 @@ class Matcha:
         quantities of WignerDGradients.get_derivatives, WignerDGradients.py:247-302).
         L defaults to L_max; angles (B,) in radians."""
         out = self.score_and_derivatives(sigma, alpha, beta, gamma, L)
-        h = out[:, 4:]
-        H = torch.stack([torch.stack([h[:, 0], h[:, 1], h[:, 2]], -1),
-                         torch.stack([h[:, 1], h[:, 3], h[:, 4]], -1),
-                         torch.stack([h[:, 2], h[:, 4], h[:, 5]], -1)], -2)
+        h = out[:, 4:].unbind(1)
+        H = torch.stack([h[i] for i in (0, 1, 2, 1, 3, 4, 2, 4, 5)], -1).view(-1, 3, 3)
         return out[:, 0], out[:, 1:4], H
 
     @torch.no_grad()
