@@ -35,9 +35,9 @@ sys.path.insert(0, ROOT)
 N_BOX, L_MAX, LI = 64, 32, [8, 16, 24]
 SHIFT_RADIUS, UPSAMPLE = 5, 8
 METRIC = "subtomograms/s at 64^3 L=32 (one alternation: FLE+sigma, SO(3) grid, Newton march, shift)"
-KERNELS_PER_STEP = 16  # FLE fold_split, gemm_tc, expand; sigma; SO(3) grid; fold_sigma, newton_march,
-# reduce_candidates; tracker_update; shift patch_fft_xy64, fft_z64, updft1_tc x2 (the Nyquist plane),
-# updft1_tc, updft23_tc, finalize_tc
+KERNELS_PER_STEP = 15  # FLE fold_split, gemm_tc, expand; sigma; SO(3) grid; fold_sigma, newton_march,
+# reduce_candidates; tracker_update; shift patch_fft_xy64, fft_z64, updft1_tc (pass 1), updft1_tc (the
+# Nyquist plane's pass 2), updft23_tc, finalize_tc
 
 
 def parse():
@@ -302,9 +302,9 @@ def kernel_work(B):
         "tracker_update_kernel": ("hbm", 3 * 4 + 2 * 32 + 36),
         "patch_fft_xy64_kernel": ("hbm", vol + spec),
         "fft_z64_kernel": ("hbm", spec + a1 + a1n),
-        "updft1_tc_kernel": ("tensor", 2.0 * (N // 2 * N) * (2 * N) * (2 * U)),
-        # the Nyquist plane m2 = N/2 as its own two small GEMMs: rows (b, m1), then rows (b, u0)
-        "updft1_tc_kernel (Nyquist plane, pass 1)": ("tensor", 2.0 * N * (2 * N) * (2 * U)),
+        # rows (b, m2 < N/2, m1) and, in the same launch, (b, m1) of the Nyquist plane m2 = N/2, whose
+        # second pass (rows (b, u0)) has its own
+        "updft1_tc_kernel": ("tensor", 2.0 * (N // 2 * N + N) * (2 * N) * (2 * U)),
         "updft1_tc_kernel (Nyquist plane, pass 2)": ("tensor", 2.0 * U * (2 * N) * (2 * U)),
         "updft23_tc_kernel": ("tensor", 2.0 * (U * N // 2) * (2 * U) * (2 * N) + 2.0 * U * U * U * (N + 2)),
         "finalize_tc_kernel": ("hbm", 16),

@@ -345,8 +345,10 @@ int mtb_shift_status(mtb_shift* h, mtb_stream_t stream);
  * groups, in a ring of the last n_calls calls (0 switches it off).  mtb_shift_profile_read
  * synchronises on the recorded events and returns in ms[0..5] the summed time of
  * (patch + xy FFT, z FFT + product, Nyquist plane, upsampled-DFT pass 1, passes 2+3,
- * finalize) over those calls and their number in *calls.  For the FP32 path the Nyquist
- * entry spans no kernel and pass 1 / passes 2+3 are its two upsampled-DFT kernels. */
+ * finalize) over those calls and their number in *calls.  The Nyquist entry is the launch of
+ * that plane's second pass beside the fused passes 2+3 (its first pass runs in pass 1's launch);
+ * with unfused passes and on the FP32 path it has none and the entry spans no kernel.  On the
+ * FP32 path pass 1 / passes 2+3 are its two upsampled-DFT kernels. */
 int mtb_shift_profile(mtb_shift* h, int n_calls);
 int mtb_shift_profile_read(mtb_shift* h, float* ms, int* calls);
 

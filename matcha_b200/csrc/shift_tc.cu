@@ -1175,7 +1175,6 @@ int shift_tc_passes(ShiftTc* t, int B, cudaStream_t st, const cudaEvent_t* marks
   const CUtensorMap& mapE1 = *reinterpret_cast<const CUtensorMap*>(t->mapE1);
   const CUtensorMap& mapA1n = *reinterpret_cast<const CUtensorMap*>(t->mapA1n);
   const CUtensorMap& mapA2n = *reinterpret_cast<const CUtensorMap*>(t->mapA2n);
-  if (marks && marks[0]) cudaEventRecord(marks[0], st);
   // pass 1: row (b, m2, m1) -> A2 row (b U + u0) HH + m2, word m1, and the Nyquist plane's row
   // (b, m1) -> A2n row b U + u0, word m1
   Pass1 p1 = pass1_params(t, B * HH * N, t->R1);
@@ -1197,6 +1196,7 @@ int shift_tc_passes(ShiftTc* t, int B, cudaStream_t st, const cudaEvent_t* marks
       nullptr, t->err);
   mtb_prof_end(st, "updft1_tc_kernel");
   MTB_LAUNCH_CHECK();
+  if (marks && marks[0]) cudaEventRecord(marks[0], st);
   // the Nyquist plane's pass 2, A2n E1 -> Y, in pass 2's launch or on its own beside the fused passes
   const Pass1 py = pass1_params(t, B * U, t->R2n);
   if (t->fused) {

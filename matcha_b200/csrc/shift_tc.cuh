@@ -38,10 +38,10 @@ struct ShiftTc {
 int shift_tc_fits(int N, int U);
 int shift_tc_prepare(ShiftTc* t, int N, int H, int U, int uf, float dftshift, int max_batch);
 void shift_tc_release(ShiftTc* t);
-// Nyquist plane, pass 1 and passes 2+3 (fused, or pass 2 then pass 3) for B subtomograms whose
+// Pass 1, the Nyquist plane and passes 2+3 (fused, or pass 2 then pass 3) for B subtomograms whose
 // pass-1 operands A1 and A1n have been written (fft_z split).
-// marks (or null): events recorded on st after the Nyquist plane's two GEMMs, pass 1 and
-// passes 2+3.
+// marks (or null): events recorded on st after pass 1 (the Nyquist plane's included), after the
+// launch of the Nyquist plane's pass 2 where it has one of its own, and after passes 2+3.
 int shift_tc_passes(ShiftTc* t, int B, cudaStream_t st, const cudaEvent_t* marks = nullptr);
 // Synchronises st; MTB_ERR_TIMEOUT if a device-side wait gave up, with the code of the
 // wait that gave up first in *site (when site is not null).
