@@ -321,27 +321,29 @@ __device__ __forceinline__ void pass(const float4* __restrict__ S, const float2*
       }
       const float2 z1 = cmulf(sm.ea[c][mp], egm);
       const float2 z2 = cmulf(eam, sm.eg[c][mp]);
-      const float r1 = z1.x * A1r[c] - z1.y * A1i[c], r2 = z2.x * A2r[c] - z2.y * A2i[c];
-      acc[c][A_VAL] += r1 + r2;
+      // which product of a pair is fused is written out, so that the one- and two-candidate kernels,
+      // and later compilers, round alike
+      auto real = [](float2 z, float r, float i) { return __fmaf_rn(z.x, r, -__fmul_rn(z.y, i)); };
+      auto imag = [](float2 z, float r, float i) { return __fmaf_rn(z.x, i, __fmul_rn(z.y, r)); };
+      auto lin = [](float x, float u, float y, float v) { return __fmaf_rn(x, u, __fmul_rn(y, v)); };
+      auto add = [](float& to, float v) { to = __fadd_rn(to, v); };
+      const float r1 = real(z1, A1r[c], A1i[c]), r2 = real(z2, A2r[c], A2i[c]);
+      add(acc[c][A_VAL], __fadd_rn(r1, r2));
       if (DERIVS) {
         const float fM = (float)mp, fm = (float)m;
-        // which product of a pair is fused is written out, so that the one- and two-candidate
-        // kernels, and later compilers, round alike
-        auto imag = [](float2 z, float r, float i) { return __fmaf_rn(z.x, i, __fmul_rn(z.y, r)); };
-        auto lin = [](float x, float u, float y, float v) { return __fmaf_rn(x, u, __fmul_rn(y, v)); };
         const float j1 = imag(z1, A1r[c], A1i[c]), j2 = imag(z2, A2r[c], A2i[c]);
-        const float q1 = z1.x * B1r[c] - z1.y * B1i[c], q2 = z2.x * B2r[c] - z2.y * B2i[c];
+        const float q1 = real(z1, B1r[c], B1i[c]), q2 = real(z2, B2r[c], B2i[c]);
         const float k1 = imag(z1, B1r[c], B1i[c]), k2 = imag(z2, B2r[c], B2i[c]);
-        const float h1 = z1.x * C1r[c] - z1.y * C1i[c], h2 = z2.x * C2r[c] - z2.y * C2i[c];
-        acc[c][A_GA] -= lin(fM, j1, fm, j2);
-        acc[c][A_GG] -= lin(fm, j1, fM, j2);
-        acc[c][A_GB] += q1 + q2;
-        acc[c][A_HAA] -= fM * fM * r1 + fm * fm * r2;
-        acc[c][A_HGG] -= fm * fm * r1 + fM * fM * r2;
-        acc[c][A_HAG] -= fM * fm * (r1 + r2);
-        acc[c][A_HAB] -= lin(fM, k1, fm, k2);
-        acc[c][A_HBG] -= lin(fm, k1, fM, k2);
-        acc[c][A_HBB] += h1 + h2;
+        const float h1 = real(z1, C1r[c], C1i[c]), h2 = real(z2, C2r[c], C2i[c]);
+        add(acc[c][A_GA], -lin(fM, j1, fm, j2));
+        add(acc[c][A_GG], -lin(fm, j1, fM, j2));
+        add(acc[c][A_GB], __fadd_rn(q1, q2));
+        add(acc[c][A_HAA], -lin(__fmul_rn(fM, fM), r1, __fmul_rn(fm, fm), r2));
+        add(acc[c][A_HGG], -lin(__fmul_rn(fm, fm), r1, __fmul_rn(fM, fM), r2));
+        acc[c][A_HAG] = __fmaf_rn(-__fmul_rn(fM, fm), __fadd_rn(r1, r2), acc[c][A_HAG]);
+        add(acc[c][A_HAB], -lin(fM, k1, fm, k2));
+        add(acc[c][A_HBG], -lin(fm, k1, fM, k2));
+        add(acc[c][A_HBB], __fadd_rn(h1, h2));
       }
     }
   }

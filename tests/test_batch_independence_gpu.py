@@ -5,7 +5,7 @@ import numpy as np
 import pytest
 import torch
 
-from tests.helpers import haar_quaternions
+from tests.helpers import haar_quaternions, synthetic_sigma
 from tests.test_prepare import _prepare_gpu
 
 pytestmark = pytest.mark.gpu
@@ -42,6 +42,24 @@ def test_norms(cuda_device, N, L):
     for B in (1, 149, 297, 593):
         assert torch.equal(fle._forward(v[:B], True)[1], whole[:B]), B
     fle.status()
+
+
+@pytest.mark.parametrize("L,Li,C,steps", [(32, [8, 16, 24], 10, 1), (64, [16, 32, 48], 4, 1), (24, [8, 16], 2, 3)])
+def test_marches_of_several_stages(cuda_device, L, Li, C, steps):
+    """One and two candidates of a subtomogram per CTA, by the number of CTAs."""
+    from matcha_b200.core.Matcha import Matcha
+
+    big = 2 * 148 // C + 2
+    sig, _ = synthetic_sigma(np.random.default_rng(L), 4, L)
+    sig = torch.from_numpy(sig).to(cuda_device)[torch.arange(big) % 4]
+    sig = sig * (1 + torch.arange(big, device=cuda_device)[:, None] / big)
+    m = Matcha(batchsize=big, device=cuda_device, L_max=L, matcha_config=dict(Li=Li, candidates=C, num_steps=steps))
+    g = torch.Generator(device=cuda_device).manual_seed(L)
+    start = torch.rand((3, big, C), generator=g, device=cuda_device) * 3
+    whole = m.march(*start, sig)
+    for B in (1, 5, big - 3):
+        for x, y in zip(m.march(*start[:, :B], sig[:B]), whole):
+            assert torch.equal(x, y[:B]), B
 
 
 @pytest.mark.parametrize("N,radius", [(16, 7.0), (64, 30.0), (90, 40.0)])
