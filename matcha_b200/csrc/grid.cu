@@ -12,8 +12,8 @@
 // twiddle matrix) is the same for the whole warp, so one broadcast 16-byte load feeds twelve or
 // six multiply-adds.  A CTA takes 256 / n beta values at a time, and a cluster of up to eight CTAs
 // shares a subtomogram's (cluster_size).  Every sum runs in the order of the general kernel in
-// search.cu with the same roundings, so both give the same grid bit by bit: near beta = 0 or pi whole
-// diagonals of the grid tie but for rounding, and the choice among them must not depend on the path.
+// search.cu with the same roundings (re_mac, im_mac): near beta = 0 or pi whole diagonals of the grid
+// tie but for rounding, and the choice among them must not depend on the path.
 //
 // Top-k: f goes to shared memory, each thread keeps its column's maximum, and a warp takes out
 // its best value while that beats the CTA's C-th best so far; the column that gave it is searched
@@ -76,15 +76,6 @@ __device__ __forceinline__ Best warp_best(Best b, int* lane) {
   return r;
 }
 
-// The complex multiply-add steps with the roundings of the general kernel's
-// re += x tx - y ty, im += x ty + y tx (one product of each pair is fused, the sum is not).
-__device__ __forceinline__ float re_mac(float a, float x, float y, float tx, float ty) {
-  return __fadd_rn(a, __fmaf_rn(x, tx, -__fmul_rn(y, ty)));
-}
-__device__ __forceinline__ float im_mac(float a, float x, float y, float tx, float ty) {
-  return __fadd_rn(a, __fmaf_rn(y, tx, __fmul_rn(x, ty)));
-}
-
 template <int L0>
 __global__ void __launch_bounds__(kGT, L0 <= 8 ? 4 : 2)
 so3_grid_columns_kernel(const float2* __restrict__ sigma, int64_t stride, const float* __restrict__ dtab, int C,
@@ -142,8 +133,8 @@ so3_grid_columns_kernel(const float2* __restrict__ sigma, int64_t stride, const 
 #pragma unroll
           for (int i = 0; i < JB; ++i) {
             const float d = j0 + i < n ? __ldg(dtab + (int64_t)(j0 + i) * nk + idx) : 0.f;
-            re[i] += d * s.x;
-            im[i] += d * s.y;
+            re[i] = fmaf(d, s.x, re[i]);
+            im[i] = fmaf(d, s.y, im[i]);
           }
         }
       }

@@ -3,6 +3,15 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+// The complex multiply-add steps re += x tx - y ty, im += x ty + y tx of both grid kernels' transforms,
+// with the roundings written out: one product of each pair is fused, the sum is not.
+__device__ __forceinline__ float re_mac(float a, float x, float y, float tx, float ty) {
+  return __fadd_rn(a, __fmaf_rn(x, tx, -__fmul_rn(y, ty)));
+}
+__device__ __forceinline__ float im_mac(float a, float x, float y, float tx, float ty) {
+  return __fadd_rn(a, __fmaf_rn(y, tx, __fmul_rn(x, ty)));
+}
+
 // Whether grid_columns_launch covers a grid: oversampling 2, 3 <= L0 <= 16.
 bool grid_columns_cover(int L0, int K);
 

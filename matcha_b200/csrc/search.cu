@@ -170,8 +170,8 @@ so3_grid_topk_kernel(const float2* __restrict__ sigma, int64_t stride, int B,
       for (int l = l0; l < L0; ++l) {
         const int idx = mtb_dsize(l - 1) + (mp + l) * (2 * l + 1) + (m + l);
         const float d = STAGED ? dj[idx] : __ldg(dj + idx);
-        re += d * sg[idx].x;
-        im += d * sg[idx].y;
+        re = fmaf(d, sg[idx].x, re);
+        im = fmaf(d, sg[idx].y, im);
       }
       F[q] = make_float2(re, im);
     }
@@ -184,8 +184,8 @@ so3_grid_topk_kernel(const float2* __restrict__ sigma, int64_t stride, int B,
       float re = 0.f, im = 0.f;
       for (int c = 0; c < P; ++c) {
         const float2 f = fr[c], t = tr[c];
-        re += f.x * t.x - f.y * t.y;
-        im += f.x * t.y + f.y * t.x;
+        re = re_mac(re, f.x, f.y, t.x, t.y);
+        im = im_mac(im, f.x, f.y, t.x, t.y);
       }
       G[q] = make_float2(re, im);
     }
@@ -214,7 +214,7 @@ so3_grid_topk_kernel(const float2* __restrict__ sigma, int64_t stride, int B,
       float re = 0.f;
       for (int r = 0; r < P; ++r) {
         const float2 gv = gc[r * n], t = ta[r];
-        re += gv.x * t.x - gv.y * t.y;
+        re = re_mac(re, gv.x, gv.y, t.x, t.y);
       }
       offer(re * inv_n2, (j0 + jb) * n * n + qq);
     }
