@@ -21,7 +21,7 @@
 // the pair (p(x), p(x + 1)), the second value from the next lane, wherever one of the two lies in
 // the mask (nothing else reads the patch), so that the rotation reads both x corners of a row in
 // one 8-byte load, and adds the masked sum and sum of squares to the subtomogram's FP64
-// statistics.  Bound by instruction issue; 1000 of 64^3 647 -> 500 us against 300 for the bytes
+// statistics.  Bound by instruction issue; 1000 of 64^3 647 -> 502 us against 300 for the bytes
 // (before: a column to a thread, both rows and both values of a pair interpolated for each voxel).
 // extract_kernel does the same voxel by voxel from global memory for boxes whose plane does not
 // fit in shared memory.
@@ -34,7 +34,7 @@
 // mask per corner.  Values are normalised as they are read: (p - mean) / std inside the mask,
 // 0 outside.  The gathers are bound by the L1 data stage, which takes about eight passes for a
 // warp-wide corner read: the pair layout halves the number of reads, and the brick's shape follows
-// the rotation, so that few source rows lie under it.  1000 of 64^3 1242 -> 943 us (before: fixed
+// the rotation, so that few source rows lie under it.  1000 of 64^3 1242 -> 959 us (before: fixed
 // 8 x 4 x 1 bricks, and a warp with shell voxels went both ways, corner by corner).
 #include <limits.h>
 #include <math.h>
@@ -109,11 +109,9 @@ __device__ __forceinline__ float patch_value(const Axis& ax, const Axis& ay, con
   return p;
 }
 
-template <int NT>
-__global__ void __launch_bounds__(kPT) extract_kernel(const float* __restrict__ vol, int n_rt,
+__global__ void __launch_bounds__(kPT) extract_kernel(const float* __restrict__ vol, int N,
                                                       const float* __restrict__ shift_xyz, int thresh,
                                                       float2* __restrict__ pairs, double* __restrict__ stats) {
-  const int N = NT ? NT : n_rt;
   __shared__ double red[2][kPT / 32];
   extern __shared__ Axis s_y[];  // the y axis of every row (N entries)
   const int z = blockIdx.x, b = blockIdx.y;
@@ -308,10 +306,10 @@ __global__ void __launch_bounds__(kPT, NT ? (BOX ? 6 : 7) : 5) rotate_kernel(con
   const float half = (N % 2 == 0) ? 0.5f * (float)N : 0.5f * (float)(N - 1);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   // The brick's extents: 8 along x, so that a row's part of the store is a whole sector (bricks of 4
-  // or 2 along x as well: 956 against 860 us), and 4 along y and z together.  A corner read touches a
+  // or 2 along x as well: 956 against 860 us, at a mask radius of 28.8), and 4 along y and z together.  A corner read touches a
   // line of L1 for about every source row (y, z) under the brick, that is, for its faces seen along
   // the source's x axis, whose components are the R0k.  A warp walks along x, where a brick finds
-  // lines of the one before it (with the warps next to each other along x instead 1258 us).
+  // lines of the one before it (with the warps next to each other along x instead 1258 us there).
   int ly = 2, lz = 0;
   constexpr int lx = 3;
   float best = 1e30f;
@@ -411,10 +409,10 @@ int launch(const float* volumes, int B, int N, const float* shift_xyz, const dou
     MTB_CUDA_TRY(cudaFuncSetAttribute(extract_staged_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       220 * 1024));
   // Where four planes a CTA still give 8 CTAs an SM, the prologues are shared by two planes in the
-  // extraction (1000 of 64^3: 583 us with one, 514 with four, 500 with two), and bricks of the rotation
-  // reach over four planes (925, 892 and 861 us with one, two and four) or, past 64^3, where the
-  // source under four planes outgrows L1, over two (100 of 96^3 423, 384 and 417 us).  Below, a plane a
-  // CTA keeps the SMs busy.
+  // extraction (1000 of 64^3: 557 us with one, 502 with two), and bricks of the rotation reach over four
+  // planes (1023, 992 and 959 us with one, two and four) or, past 64^3, where the source under four
+  // planes outgrows L1, over two (100 of 96^3 413, 412 and 452 us, 300 of 80^3 753, 703 and 746).  Below,
+  // a plane a CTA keeps the SMs busy.
   const bool wide = (int64_t)B * ((N + 3) / 4) >= 148 * 8;
   const int planes = wide ? 2 : 1, lz_max = wide ? (N <= 64 ? 2 : 1) : 0;
   mtb_prof_begin(st);
@@ -422,8 +420,7 @@ int launch(const float* volumes, int B, int N, const float* shift_xyz, const dou
     extract_staged_kernel<NT><<<dim3((N + planes - 1) / planes, B), kPT, ext_smem, st>>>(
         volumes, N, planes, shift_xyz, thresh, work, stats);
   else
-    extract_kernel<NT><<<dim3(N, B), kPT, (size_t)N * sizeof(Axis), st>>>(volumes, N, shift_xyz, thresh, work,
-                                                                          stats);
+    extract_kernel<<<dim3(N, B), kPT, (size_t)N * sizeof(Axis), st>>>(volumes, N, shift_xyz, thresh, work, stats);
   mtb_prof_end(st, "extract_kernel");
   MTB_LAUNCH_CHECK();
   const dim3 grid((N + (1 << lz_max) - 1) >> lz_max, B);
