@@ -109,6 +109,10 @@ __device__ __forceinline__ float patch_value(const Axis& ax, const Axis& ay, con
   return p;
 }
 
+// Boxes whose plane does not fit in shared memory: a warp walks rows, 31 columns at a time (the 32nd
+// lane's value is only the last pair's second), the eight corners of a voxel from global memory.  Bound
+// by the latency of those reads; 4 of 240^3 487 us with both values of a pair read by its thread, 573
+// with the pairs before the mask's first column beside them, 290 so.
 __global__ void __launch_bounds__(kPT) extract_kernel(const float* __restrict__ vol, int N,
                                                       const float* __restrict__ shift_xyz, int thresh,
                                                       float2* __restrict__ pairs, double* __restrict__ stats) {
@@ -123,30 +127,32 @@ __global__ void __launch_bounds__(kPT) extract_kernel(const float* __restrict__ 
   __syncthreads();
   const Axis az = patch_axis(z, sz, N);
   const float* pl[2] = {v + (int64_t)az.j0 * NN, v + (int64_t)az.j1 * NN};
-  const int c = N / 2;
-  const int dz2 = (z - c) * (z - c);
-  const int TXW = N < kPT ? N : kPT, RP = kPT / TXW;
-  const int xi = threadIdx.x % TXW, yi = threadIdx.x / TXW;
+  const int c = N / 2, rem = thresh - (z - c) * (z - c);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int rows = (N + kPT / 32 - 1) / (kPT / 32), y0 = warp * rows, y1 = min(y0 + rows, N);
   float s1 = 0.f, s2 = 0.f;
-  if (yi < RP) {
-    for (int x = xi; x < N; x += TXW) {
-      const Axis ax = patch_axis(x, sx, N), ax1 = patch_axis(x + 1, sx, N);
-      const int dx2 = (x - c) * (x - c);
-      for (int y = yi; y < N; y += RP) {
-        const int dzy2 = dz2 + (y - c) * (y - c);
-        const bool in0 = dzy2 + dx2 < thresh, in1 = x + 1 < N && dzy2 + (x + 1 - c) * (x + 1 - c) < thresh;
-        if (!in0 && !in1) continue;
+  for (int x0 = 0; x0 < N; x0 += 31) {
+    const bool last = x0 + 32 >= N, own = lane < 31 || last;
+    const int x = x0 + lane;
+    const Axis ax = patch_axis(x, sx, N);
+    const int d0 = x < N ? (x - c) * (x - c) : 1 << 24, d1 = x + 1 < N ? (x + 1 - c) * (x + 1 - c) : 1 << 24;
+    for (int y = y0; y < y1; ++y) {
+      const int ry = rem - (y - c) * (y - c);
+      const bool in0 = d0 < ry, write = min(d0, d1) < ry;
+      if (!__any_sync(0xffffffffu, write)) continue;
+      float p = 0.f;
+      if (write) {
         const Axis ay = s_y[y];
-        auto at = [&](int k, int row, int col) { return __ldg(pl[k] + (int64_t)row * N + col); };
-        const float p = patch_value(ax, ay, az, at);
-        const float p1 = x + 1 < N ? patch_value(ax1, ay, az, at) : 0.f;
-        out[(int64_t)y * N + x] = make_float2(p, p1);
-        if (in0) {
-          s1 += p;
-          s2 = fmaf(p, p, s2);
-        }
+        p = patch_value(ax, ay, az, [&](int k, int row, int col) { return __ldg(pl[k] + (int64_t)row * N + col); });
+      }
+      const float p1 = __shfl_down_sync(0xffffffffu, p, 1);
+      if (own && write) out[(int64_t)y * N + x] = make_float2(p, x + 1 < N ? p1 : 0.f);
+      if (own && in0) {
+        s1 += p;
+        s2 = fmaf(p, p, s2);
       }
     }
+    if (last) break;
   }
   block_add(s1, s2, stats + 2 * b, red);
 }
