@@ -188,9 +188,9 @@ gemm_fp32_kernel(const float* __restrict__ A, int64_t a_stride_class, int M, int
 // with the sign in bit 0 (-1: no imaginary part).  The work is a gather of a row that L1 holds, so
 // latency sets the time: a cluster of CTAs shares a subtomogram's coefficients and a thread has four
 // in flight.  The sum of squares is formed by `slices` of the coefficients, whose number depends on
-// ne alone and which the CTAs take in turn, so that a norm does not depend on the batch; their
-// warps' sums meet through distributed shared memory in a fixed order.  100 subtomograms of 96^3
-// 18 us, one of 48^3 9 us.
+// ne alone and which the CTAs take in turn, so that a norm does not depend on the batch; the slices'
+// sums meet through distributed shared memory in order.  100 subtomograms of 96^3 18 us, one of 48^3
+// 9 us.
 constexpr int kET = 256, kSlices = 8;
 
 __device__ __forceinline__ float signed_at(const float* c, int code) {
@@ -206,7 +206,7 @@ expand_kernel(const float* __restrict__ C, int64_t c_ld, int ne, int slices, con
   const int rank = (int)cluster.block_rank(), parts = (int)cluster.num_blocks(), b = blockIdx.y;
   const float* c = C + (int64_t)b * c_ld;
   float2* o = out + (int64_t)b * out_stride;
-  __shared__ float red[kSlices][kET / 32];
+  __shared__ float red[kSlices][kET / 32], total[kSlices];
   const int step = slices * kET;
   for (int s = rank; s < slices; s += parts) {
     float ss = 0.f;
@@ -227,18 +227,17 @@ expand_kernel(const float* __restrict__ C, int64_t c_ld, int ne, int slices, con
     if ((threadIdx.x & 31) == 0) red[s][threadIdx.x >> 5] = ss;
   }
   if (!norms) return;  // the same for the whole cluster
+  __syncthreads();
+  if (threadIdx.x < slices && (threadIdx.x & (parts - 1)) == rank) {
+    float s = 0.f;
+    for (int w = 0; w < kET / 32; ++w) s += red[threadIdx.x][w];
+    total[threadIdx.x] = s;
+  }
   cluster.sync();
-  if (rank == 0 && threadIdx.x < 32) {
-    constexpr int kW = kET / 32, kEach = kSlices * kW / 32;  // sums of all slices' warps, kEach to a lane
-    double sum = 0.0;
-#pragma unroll
-    for (int j = 0; j < kEach; ++j) {
-      const int e = j * 32 + (int)threadIdx.x, s = e / kW;
-      if (s < slices) sum += cluster.map_shared_rank(&red[s][e % kW], s & (parts - 1))[0];
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-    if (threadIdx.x == 0) norms[b] = sqrtf((float)sum);
+  if (rank == 0 && threadIdx.x == 0) {
+    float sum = 0.f;
+    for (int s = 0; s < slices; ++s) sum += cluster.map_shared_rank(&total[s], s & (parts - 1))[0];
+    norms[b] = sqrtf(sum);
   }
   cluster.sync();  // no CTA leaves while its sums are read
 }
