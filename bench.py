@@ -286,6 +286,7 @@ def kernel_work(B):
     per launch of B subtomograms, amount in bytes for "hbm" and FLOP for "tensor"/"fp32"."""
     N, H, U = N_BOX, N_BOX // 2 + 1, int(np.ceil(UPSAMPLE * (2 * SHIFT_RADIUS + 1)))
     n_rep, n_cols, ne = 15216, 8252, 8252
+    n_ball = 113081                      # voxels of the radius-30 ball: what the expansion reads of a volume
     vol = 4 * N ** 3                     # one float32 subtomogram
     spec = 8 * N * N * H                 # (N, N, N/2+1) complex64 plane transforms
     a1 = 2 * 2 * (N // 2) * N * 2 * N    # pass-1 operand: rows (m2 < N/2, m1), K (m0, re/im), bf16 hi and lo
@@ -293,7 +294,7 @@ def kernel_work(B):
     a2 = 2 * 2 * U * (N // 2) * 2 * N    # pass-2 operand: rows (u0, m2 < N/2), K (m1, re/im), hi and lo
     dsize = lambda L: (L + 1) * (2 * L + 1) * (2 * L + 3) // 3
     work = {
-        "fold_split_kernel": ("hbm", vol + 2 * 2 * 8 * n_rep),
+        "fold_split_kernel": ("hbm", 4 * n_ball + 2 * 2 * 8 * n_rep),
         "gemm_tc_kernel": ("tensor", 2.0 * n_rep * n_cols),
         "expand_kernel": ("hbm", 4 * n_cols + 8 * ne),
         "sigma_kernel": ("hbm", 8 * ne + 8 * dsize(L_MAX)),
@@ -366,10 +367,11 @@ def kernel_table(prof, steps, B, peaks, fp32_peak):
 
 
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per subtomogram of the shift kernels,
-# from one ncu capture at 200 subtomograms (profiles/shift_64_uf8_b200.md), scaled to a launch by
-# the subtomograms it processes (their traffic grows in proportion to the batch)
-DRAM_BYTES_PER_SUBTOMO = {"patch_fft_xy64_kernel": 1_910_000, "fft_z64_kernel": 2_085_000,
-                          "updft1_tc_kernel": 2_205_000, "updft23_tc_kernel": 1_525_000}
+# from ncu captures at 200 subtomograms (profiles/stages_64_L32_b200.md; pass 1, whose launch was not
+# in it, profiles/shift_64_uf8_b200.md), scaled to a launch by the subtomograms it processes (their
+# traffic grows in proportion to the batch)
+DRAM_BYTES_PER_SUBTOMO = {"patch_fft_xy64_kernel": 1_905_000, "fft_z64_kernel": 1_880_000,
+                          "updft1_tc_kernel": 2_205_000, "updft23_tc_kernel": 1_520_000}
 
 
 # ---------------------------------------------------------------- ranks

@@ -69,9 +69,11 @@ typedef struct mtb_search mtb_search;
 int mtb_search_create(const mtb_search_config* cfg, mtb_search** out);
 void mtb_search_destroy(mtb_search* h);
 
-/* Host-only query of the grid kernel's pass shape for (L0, K) (no counterpart in the
+/* Host-only query of the general grid kernel's pass shape for (L0, K) (no counterpart in the
  * reference): beta values per pass, whether their d-table rows are staged in shared memory,
- * and its dynamic shared memory.  MTB_ERR_ARG when the grid does not fit shared memory. */
+ * and its dynamic shared memory.  MTB_ERR_ARG when the grid does not fit shared memory.  It
+ * decides which (L0, K) are taken; those of K = 2 with 3 <= L0 <= 16 run the column kernel, whose
+ * shapes are fixed at compile time. */
 int mtb_so3_grid_plan(int L0, int K, int* beta_per_pass, int* staged, int64_t* smem);
 
 /* Grid search: f(beta_j, alpha_a, gamma_g) on the (2 L0 K)^3 grid, top-`candidates`

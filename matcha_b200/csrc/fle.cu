@@ -251,7 +251,7 @@ expand_kernel(const float* __restrict__ C, int64_t c_ld, int ne, int slices, con
 // K is small (4.5 on average at 64^3), so instruction issue bounds it, with the operand loads, the
 // row pointers and the stores beside the products: a thread takes 4 rows x 3 columns (4 x 1 284 us, 4 x
 // 2 263, 4 x 4 276, 4 x 3 255; 1000 subtomograms of 64^3, 0.85 GB of outputs, 128 us at the copy's
-// rate), and 64 registers, for eight CTAs of 128 threads an SM, 221 us.  100 of 96^3 156 -> 101 us.
+// rate), and 64 registers, for eight CTAs of 128 threads an SM, 226 us.  100 of 96^3 156 -> 106 us.
 constexpr int kSC = 3, kSigmaT = 128;
 
 __global__ void __launch_bounds__(kSigmaT, 8)

@@ -11,12 +11,11 @@
 //                products: the same bytes per stage, two thirds of the bytes per product, and B_hi
 //                read once instead of twice.  (With stages of 64 along K only two fit, which was
 //                1242 against 1187 us for 100 of 96^3 and 2.2x slower for 1000 of 64^3.)
-// The second is for a basis past 1 GB (80^3: 2 GB), where the loads, into shared memory and from
-// DRAM, set the pace.  Below, the first: it adds the same chunks in the same order however the tiles
-// are cut, so that the coefficients keep their bits, and with them the orientation search its
-// choice between equal scores (the angles at beta = 0, alpha at 0 or 2 pi), which any rounding
-// moves; at 64^3 (500 MB) the second would save 15 to 30 % of the GEMM (1000 subtomograms 550
-// against 648 us).  Times of the GEMM, before (segmented, one CTA per tile) and now: 100 of 96^3
+// The second is for a basis past 1 GB (80^3: 2 GB).  That line is not where it stops being the faster:
+// at 64^3 (500 MB) it would save 15 to 30 % of the GEMM too (1000 subtomograms 550 against 648 us).
+// It is drawn for last bits.  The orientation search's choice between equal scores (the angles at
+// beta = 0, alpha at 0 or 2 pi) follows them, and up to 64^3 the coefficients keep those of the
+// segmented order; past it, where the loads take twice the products' time, they got others.  Times of the GEMM, before (segmented, one CTA per tile) and now: 100 of 96^3
 // 1397 -> 1105 us (5.5 TB/s of basis), 128 of 80^3 647 -> 381 us, 1000 of 64^3 679 -> 648 us, 256 of
 // 64^3 321 -> 237 us, one of 64^3 291 -> 144 us, 128 of 48^3 138 -> 66 us, one of 48^3 118 -> 38 us.
 //

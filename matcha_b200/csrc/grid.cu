@@ -255,6 +255,7 @@ template <int L0>
 int launch(const float2* sigma, int64_t stride, int B, const float* dtab, int C, float* a, float* b, float* g,
            float* grid, cudaStream_t st) {
   using S = Shape<L0>;
+  static_assert(S::smem + (kWarps + 2) * kCmax * sizeof(Best) + S::n * sizeof(float2) <= kSmemOptIn, "shared memory");
   MTB_CUDA_TRY(cudaFuncSetAttribute(so3_grid_columns_kernel<L0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)S::smem));
   constexpr int npass = (S::n + S::JB - 1) / S::JB;

@@ -191,7 +191,7 @@ __device__ __forceinline__ float2 cmulf(float2 a, float2 b) {
 // the recurrence factors; their d, d', d'' run side by side.  FOLDED reads the folded sigma S
 // of this subtomogram; otherwise each step folds the four images from sigma itself.
 //
-// Issue bounds it, and of the 24 M thread instructions a subtomogram took at L = 32 only a third
+// Issue and the latency of its L2 loads bound it, and of the 24 M thread instructions a subtomogram took at L = 32 only a third
 // were FP32; so everything around the chain steps is kept short: the points' trigonometry and the
 // FP64 step are one thread's, tables hold k >= 0 and are filled by all threads, offsets are 32-bit,
 // the sums of a warp are exchanged by halves.  March of 1000 subtomograms at L = 32 1104 -> 884 us,

@@ -70,8 +70,8 @@ struct GridPlan {
 
 // The pass shape: the most CTAs per SM first (the kernel is latency-bound: a CTA runs its
 // passes one after another, three barriers each), then the most beta values per pass (fewer
-// passes), then staged rows.  At L0 = 16 this is two unstaged rows, two CTAs per SM (staged,
-// the two rows take 150 KB and leave one).
+// passes), then staged rows.  (Which grids are taken is decided by it for every (L0, K), also where
+// the column kernel then runs.)
 GridPlan grid_plan(int L0, int K) {
   GridPlan best{0, true};
   int best_c = 0;
