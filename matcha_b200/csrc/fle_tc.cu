@@ -15,9 +15,10 @@
 // at 64^3 (500 MB) it would save 15 to 30 % of the GEMM too (1000 subtomograms 550 against 648 us).
 // It is drawn for last bits.  The orientation search's choice between equal scores (the angles at
 // beta = 0, alpha at 0 or 2 pi) follows them, and up to 64^3 the coefficients keep those of the
-// segmented order; past it, where the loads take twice the products' time, they got others.  Times of the GEMM, before (segmented, one CTA per tile) and now: 100 of 96^3
-// 1397 -> 1105 us (5.5 TB/s of basis), 128 of 80^3 647 -> 381 us, 1000 of 64^3 679 -> 648 us, 256 of
-// 64^3 321 -> 237 us, one of 64^3 291 -> 144 us, 128 of 48^3 138 -> 66 us, one of 48^3 118 -> 38 us.
+// segmented order; past it, where that order's loads take twice the products' time, they got others.
+// Times of the GEMM, before (segmented, one CTA per tile) and now: 100 of 96^3 1397 -> 1105 us (5.5 TB/s
+// of basis), 128 of 80^3 647 -> 381 us, 1000 of 64^3 679 -> 648 us, 256 of 64^3 321 -> 237 us, one of
+// 64^3 291 -> 144 us, 128 of 48^3 138 -> 66 us, one of 48^3 118 -> 38 us.
 //
 // Accumulation: the tensor core adds each K=16 product into the FP32 accumulator with a
 // truncating alignment, an error of about one unit in the last place of the accumulator per

@@ -28,7 +28,7 @@
 //
 // rotate_kernel: CTA = (one or four output planes z, subtomogram b), a warp = a brick of 32 voxels.
 // The sample point of output voxel v is R (v - c) + c (c = N / 2, the centre of the odd-padded
-// linspace(-1, 1) grid), so |s - c| = |v - c|: voxels farther than radius + 1.74 from c read only
+// linspace(-1, 1) grid), so |s - c| = |v - c|: voxels farther than radius + 2 from c read only
 // masked-out corners and are written as zero without loads, voxels nearer than radius - 1.74
 // read only corners inside the mask (four pair loads), and only the shell between tests the
 // mask per corner.  Values are normalised as they are read: (p - mean) / std inside the mask,
@@ -470,8 +470,9 @@ extern "C" int mtb_prepare_subtomos(const float* volumes, int B, int N, const fl
   MTB_ARG_CHECK(count > 0, "the mask is empty");
   // A rotation keeps |s - c| = |v - c|, and the corners of s lie within sqrt(3) < 1.74 of it: beyond
   // r + 1.74 all corners are outside the mask, within r - 1.74 all are inside.  What is left covers
-  // the rounding of s (1e-4 at 512).
-  const int skip2 = (int)ceil((r + 1.74) * (r + 1.74));
+  // the rounding of s (1e-4 at 512).  The outer limit is r + 2: the shell in between is empty sums over
+  // the deviation, zero, but not a number, as the mask is, where a subtomogram has no deviation.
+  const int skip2 = (int)ceil((r + 2.0) * (r + 2.0));
   const int inner2 = r > 1.74 ? (int)floor((r - 1.74) * (r - 1.74)) : 0;
   // the mask stays inside the box when every offset d with d^2 < r^2 is at most min(c, N-1-c)
   const int reach = c < N - 1 - c ? c : N - 1 - c;
