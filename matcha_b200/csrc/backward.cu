@@ -203,7 +203,7 @@ score_backward_kernel(const float2* __restrict__ sigma, int64_t stride, int L, c
 // The partial sums meet in shared memory, then through distributed shared memory, in a fixed
 // order: deterministic, and no workspace.  The rows of V of n_sub subtomograms are gathered at a
 // time (kidx: rows mu = -l..l of kpad[l] entries, -1 padded), so a barrier covers n_sub of them.
-// 256 subtomograms at L = 32 (98 MB of G): 102 us, against 2487 us for one CTA per degree
+// 256 subtomograms at L = 32 (98 MB of G): 84 us, against 2487 us for one CTA per degree
 // that walked the batch alone.
 constexpr int kBC = 32;   // columns
 constexpr int kBK = 8;    // radial entries of a warp
@@ -286,8 +286,8 @@ sigma_backward_template_kernel(const float2* __restrict__ aV, int64_t v_stride, 
           }
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
-            const int row = r + j * nrg < R ? r + j * nrg : r;
-            const float4* v4 = reinterpret_cast<const float4*>(bsm + row * ks + kt * kBK);
+            if (r + j * nrg >= R) break;
+            const float4* v4 = reinterpret_cast<const float4*>(bsm + (r + j * nrg) * ks + kt * kBK);
 #pragma unroll
             for (int k = 0; k < kBK / 2; ++k) {
               const float4 v = v4[k];

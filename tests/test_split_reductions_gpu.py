@@ -148,3 +148,24 @@ def test_template_gradient_of_few(cuda_device, B):
 
     want = sum(grad(slice(b, b + 1)) for b in range(B))
     assert (grad(slice(0, B)) - want).abs().max() < 2e-6 * want.abs().max()
+
+
+@pytest.mark.parametrize("B", [1, 9])
+def test_template_gradient_of_an_infinite_coefficient(cuda_device, B):
+    """An infinite coefficient makes its own entries infinite, not all that rows past the end touch."""
+    from matcha_b200.autograd import template_sigma
+    from matcha_b200.core.CrossCorrelationMatcher import CrossCorrelationMatcher
+    from matcha_b200.core.fle_tables import sht_index
+
+    cc = CrossCorrelationMatcher(N=16, device=cuda_device, batchsize=B, bandlimit=8, radius=7, precision="fp32")
+    cc.expand(torch.ones((B, 16, 16, 16), device=cuda_device))
+    cc._coeffs.fill_(1.0 + 1.0j)
+    at = int(cc.fle.idlm_list[0][sht_index(0)][0])
+    cc._coeffs[0, at] = complex(float("inf"), 1.0)
+    t = torch.ones((cc.fle.ne + 1,), device=cuda_device, dtype=torch.complex64, requires_grad=True)
+    template_sigma(t, cc, 1).backward(torch.full((B, 1 + 9), 1.0 + 1.0j, device=cuda_device, dtype=torch.complex64))
+    grad = torch.view_as_real(t.grad)
+    assert torch.isinf(grad[at]).all()
+    others = torch.ones(cc.fle.ne + 1, dtype=torch.bool, device=cuda_device)
+    others[at] = False
+    assert torch.isfinite(grad[others]).all()
