@@ -40,5 +40,3 @@ def test_stages_hold_their_launches(cuda_device, N, uf, r):
     assert ms["updft_pass1"] >= kernels["updft1_tc_kernel"] - slack
     assert ms["updft_pass23"] >= sum(v for k, v in kernels.items() if k.startswith("updft")
                                      and k != "updft1_tc_kernel") - slack
-    # and no stage holds another's: the nearest of them is several times longer than the slack
-    assert ms["updft_pass1"] < kernels["updft1_tc_kernel"] + 0.5 * (nyquist or 1.0) + slack
